@@ -115,7 +115,7 @@ VT_API int vt_diag_set_trace_form(vt_context* ctx, int32_t form);
 
 /* Tuning of the wavefront form's DDA kernel (values <= 0, and refill_min
  * < 0, keep their setting): queue_chunk queue records a warp takes with one
- * atomic (a multiple of 32 in [32, 1024], default 128); refill_min: a warp
+ * atomic, at most (a multiple of 32 in [32, 1024], default 64); refill_min: a warp
  * stops stepping and starts its lanes' next segments as soon as fewer than
  * refill_min of its lanes still step (checked every fourth step; 0, the
  * default, refills only every trace_steps steps).  Results are identical

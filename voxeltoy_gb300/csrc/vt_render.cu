@@ -497,16 +497,27 @@ struct GridHold<WfOneJob> {
 };
 
 // One round of tracing: every queued segment runs its DDA to the end.  Each
-// warp takes chunks of P.trace_chunk queue records with one atomic and hands
-// them to its lanes; every lane keeps the record of its next segment loaded
-// while it steps the current one, so starting a segment never waits on
-// memory, and lanes pick up a new segment every kTraceSteps steps as theirs
-// finish (with kVote also as soon as fewer than P.refill_min lanes step).
-// Resident blocks the trace kernel is compiled for: six with one job (its
-// grid record is constant), five with a job table, whose per-lane grid
-// record would otherwise spill at six blocks' 40 registers.
+// warp takes chunks of queue records with one atomic and hands them to its
+// lanes; every kTraceSteps steps (with kVote also as soon as fewer than
+// P.refill_min lanes step) the lanes whose segments ended take the next ones.
+// What bounds it is issue: 33 or so warp instructions a step, and per refill
+// the record read and the segment set-up at the efficiency of the lanes that
+// need one.  So the refill is short: no second record is kept loaded per lane
+// (eight registers; the warps that then fit hide the read instead), the chunk
+// hand-out is straight-line, and an end inside the volume is packed without
+// clamps.  A chunk is P.trace_chunk records, but no more than leaves every
+// warp four turns, down to 32: with 128 always, a queue of half a million
+// records kept two thirds of the warps busy.  Measured with the prefetched
+// records and fixed chunks before -> now (2 lanes, 8M slots): 1024^2 x 256 spp
+// of 256^3 noise 134 -> 123 ms, 1024^2 x 16 spp of a 1024^3 shell 23.7 -> 19.9
+// ms, 256^2 x 16 spp of 64^3 spheres 0.86 -> 0.72 ms, 512^2 x 1 spp 1.13 ->
+// 0.94 ms.
+// Resident blocks the trace kernel is compiled for: eight with one job (its
+// grid record is constant; 32 registers, no spill; six blocks measure 126 and
+// 20.6 ms on the two large frames), five with a job table, whose per-lane grid
+// record would otherwise spill.
 template <class Tab> struct TraceBlocks { static constexpr int value = 5; };
-template <> struct TraceBlocks<WfOneJob> { static constexpr int value = 6; };
+template <> struct TraceBlocks<WfOneJob> { static constexpr int value = 8; };
 
 template <bool kCount, int kTraceSteps, bool kVote, bool k444, class Tab>
 __global__ void __launch_bounds__(256, TraceBlocks<Tab>::value) k_wf_trace(const WfParams P, const __grid_constant__ Tab T, int par) {
@@ -521,49 +532,47 @@ __global__ void __launch_bounds__(256, TraceBlocks<Tab>::value) k_wf_trace(const
   Cnt<kCount> cnt;
 #pragma unroll
   for (int i = 0; i < C_NUM; ++i) cnt.c[i] = 0;
-  uint32_t pool = 0, pool_end = 0;
-  bool exhausted = false, have = false, have_next = false;
-  float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+  const uint32_t chunk = min(P.trace_chunk, max(32u, n / (gridDim.x * 32u) & ~31u));   // eight warps a block
+  uint32_t pool = 0, pool_end = 0;   // the rest of this warp's chunk of queue records
+  bool have = false, more = true;    // more: the queue may hold another chunk
   GridHold<Tab> gh;
   Dda s;
   uint32_t tag = 0;   // position << 1 | kind of the current segment
   for (;;) {
-    if (!have && have_next) {            // start the prefetched segment
-      have_next = false;
-      tag = __float_as_uint(nb.z);
-      if (tag != kNoSegment) {
-        gh.set(P, T, __float_as_uint(nb.w));
-        dda_begin_rec(gh.get(T), s, mk3(na.x, na.y, na.z), mk3(na.w, nb.x, nb.y));
-        if (s.state == DDA_RUNNING) have = true;
-        else P.hits[(size_t)(tag & 1u) * P.n_slots + (tag >> 1)] = pack_end(s.x, s.y, s.z, s.state);
-      }
-    }
-    unsigned need = __ballot_sync(FULL, !have_next);
-    while (need && !exhausted) {          // prefetch next records
-      if (pool >= pool_end) {
+    const unsigned need = __ballot_sync(FULL, !have);
+    if (need) {   // idle lanes take the next records
+      const uint32_t avail = pool_end - pool, want = __popc(need), r = __popc(need & lt);
+      uint32_t rec = r < avail ? pool + r : n;
+      pool += min(want, avail);
+      if (want > avail && more) {
         uint32_t c = 0;
-        if (lane == 0) c = atomicAdd(&P.ctl[ctl_index(par, CTL_QHEAD)], P.trace_chunk);
+        if (lane == 0) c = atomicAdd(&P.ctl[ctl_index(par, CTL_QHEAD)], chunk);
         c = __shfl_sync(FULL, c, 0);
-        if (c >= n) { exhausted = true; break; }
-        pool = c;
-        pool_end = min(c + P.trace_chunk, n);
+        more = c < n;
+        if (more) {
+          if (r >= avail) rec = c + (r - avail);   // within the chunk: it holds 32 records or more
+          pool_end = min(c + chunk, n);
+          pool = min(c + (want - avail), pool_end);
+        }
       }
-      const uint32_t avail = pool_end - pool;
-      const uint32_t r = __popc(need & lt);
-      if (!have_next && r < avail) {
-        na = __ldg(&q[2 * (size_t)(pool + r)]);
-        nb = __ldg(&q[2 * (size_t)(pool + r) + 1]);
-        have_next = true;
+      if (!have && rec < n) {
+        const float4 na = __ldg(&q[2 * (size_t)rec]), nb = __ldg(&q[2 * (size_t)rec + 1]);
+        tag = __float_as_uint(nb.z);
+        if (tag != kNoSegment) {
+          gh.set(P, T, __float_as_uint(nb.w));
+          dda_begin_rec(gh.get(T), s, mk3(na.x, na.y, na.z), mk3(na.w, nb.x, nb.y));
+          if (!kCount && k444 && s.state == DDA_RUNNING) dda_end_stuck(gh.get(T), s);
+          if (s.state == DDA_RUNNING) have = true;
+          else P.hits[(size_t)(tag & 1u) * P.n_slots + (tag >> 1)] = pack_end(s.x, s.y, s.z, s.state);
+        }
       }
-      pool += min(avail, (uint32_t)__popc(need));
-      need = __ballot_sync(FULL, !have_next);
+      if (!__any_sync(FULL, have) && !more && pool >= pool_end) break;
     }
-    if (__ballot_sync(FULL, have || have_next) == 0u) break;
     if (have) {
       if constexpr (!kCount && k444) dda_steps_444<kVote>(gh.get(T), s, kTraceSteps, P.refill_min);
       else dda_steps<kCount, kVote, k444>(gh.get(T), s, kTraceSteps, cnt, P.refill_min);
       if (s.state != DDA_RUNNING) {
-        P.hits[(size_t)(tag & 1u) * P.n_slots + (tag >> 1)] = pack_end(s.x, s.y, s.z, s.state);
+        P.hits[(size_t)(tag & 1u) * P.n_slots + (tag >> 1)] = pack_end_inside(s.x, s.y, s.z, s.state);
         have = false;
       }
     }
@@ -629,6 +638,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_trace_pool(const WfParams P, cons
         GridHold<Tab> tg;
         tg.set(P, T, tjob);
         dda_begin_rec(tg.get(T), t, mk3(a.x, a.y, a.z), mk3(a.w, b.x, b.y));
+        if (!kCount && k444 && t.state == DDA_RUNNING) dda_end_stuck(tg.get(T), t);
         run = t.state == DDA_RUNNING;
         if (!run) P.hits[(size_t)(ttag & 1u) * P.n_slots + (ttag >> 1)] = pack_end(t.x, t.y, t.z, t.state);
       }

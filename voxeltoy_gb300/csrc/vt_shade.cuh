@@ -311,24 +311,34 @@ VT_D SegRec seg_rec(const Frame& F, v3 o, v3 d) {
   r.inc = mk3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
   return r;
 }
-// dda_begin from a SegRec: the rest of its operations on the same values.
+VT_D bool voxel_inside(const Grid& g, int x, int y, int z) {
+  return (unsigned)x < (unsigned)g.rx && (unsigned)y < (unsigned)g.ry && (unsigned)z < (unsigned)g.rz;
+}
+// dda_begin from a SegRec: the rest of its operations on the same values
+// (a component's sign from the reciprocal, sign(d)/d as its magnitude).
 VT_D void dda_begin_rec(const Grid& g, Dda& s, v3 vo, v3 inc) {
   const v3 vp = mk3(floorf(vo.x), floorf(vo.y), floorf(vo.z));
   s.x = (int32_t)vp.x; s.y = (int32_t)vp.y; s.z = (int32_t)vp.z;
   s.steps = 0;
   s.cb = -1;
   s.bits = 0ull;
-  if (vp.x < 0.0f || vp.y < 0.0f || vp.z < 0.0f || vp.x >= (float)g.rx || vp.y >= (float)g.ry ||
-      vp.z >= (float)g.rz) {
-    s.state = DDA_MISS;
-    return;
-  }
-  s.state = DDA_RUNNING;
-  const v3 sg = mk3(inc.x > 0.0f ? 1.0f : -1.0f, inc.y > 0.0f ? 1.0f : -1.0f, inc.z > 0.0f ? 1.0f : -1.0f);
-  const v3 dis = (((vp - vo) + mk3(0.5f, 0.5f, 0.5f)) + sg * 0.5f) * inc;
+  s.state = voxel_inside(g, s.x, s.y, s.z) ? DDA_RUNNING : DDA_MISS;   // conversions saturate
+  const v3 dis = (((vp - vo) + mk3(0.5f, 0.5f, 0.5f)) +
+                  mk3(copysignf(0.5f, inc.x), copysignf(0.5f, inc.y), copysignf(0.5f, inc.z))) * inc;
   s.dx = dis.x; s.dy = dis.y; s.dz = dis.z;
-  s.ax = sg.x * inc.x; s.ay = sg.y * inc.y; s.az = sg.z * inc.z;
-  s.sx = (int32_t)sg.x; s.sy = (int32_t)sg.y; s.sz = (int32_t)sg.z;
+  s.ax = fabsf(inc.x); s.ay = fabsf(inc.y); s.az = fabsf(inc.z);
+  s.sx = inc.x > 0.0f ? 1 : -1; s.sy = inc.y > 0.0f ? 1 : -1; s.sz = inc.z > 0.0f ? 1 : -1;
+}
+
+// A segment whose origin is not a number along any axis has no crossing
+// distance and never moves: the step cap of dda.h:98 ends it where it starts,
+// a hit if that voxel is occupied.  The loop without a step count
+// (dda_steps_444) must not be entered with it.
+VT_D void dda_end_stuck(const Grid& g, Dda& s) {
+  if (s.dx == s.dx || s.dy == s.dy || s.dz == s.dz) return;
+  const int b = (s.x >> g.shx) + g.bx * (s.y >> g.shy) + g.bxy * (s.z >> g.shz);
+  const unsigned long long w = __ldg(&g.bricks[b]);
+  s.state = ((w >> brick_bit(s.x, s.y, s.z, g.shx, g.shxy, g.mx, g.my, g.mz)) & 1ull) ? DDA_HIT : DDA_MISS;
 }
 
 // DDA loop (dda.h:38-57): at most `budget` iterations of
@@ -468,6 +478,13 @@ VT_D unsigned long long pack_end(int x, int y, int z, int state) {
   z = min(max(z, -(1 << 19)), (1 << 19) - 1);
   return ((unsigned long long)((uint32_t)x & 0x1fffffu)) | ((unsigned long long)((uint32_t)y & 0x1fffffu) << 21) |
          ((unsigned long long)((uint32_t)z & 0xfffffu) << 42) | ((unsigned long long)(uint32_t)state << 62);
+}
+// pack_end of a position from -1 to the extent (every segment that started
+// inside the volume ends on one).
+VT_D unsigned long long pack_end_inside(int x, int y, int z, int state) {
+  const uint32_t lo = ((uint32_t)x & 0x1fffffu) | ((uint32_t)y << 21);
+  const uint32_t hi = (((uint32_t)y & 0x1fffffu) >> 11) | (((uint32_t)z & 0xfffffu) << 10) | ((uint32_t)state << 30);
+  return ((unsigned long long)hi << 32) | lo;
 }
 VT_D SegEnd unpack_end(unsigned long long w) {
   SegEnd e;
