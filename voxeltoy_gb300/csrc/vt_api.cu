@@ -203,6 +203,7 @@ void vt::release_context(vt_context* ctx) {
   ctx->release(ctx->d_grids);
   ctx->release(ctx->wf_mem);
   ctx->release(ctx->sbuf);
+  ctx->release(ctx->block_state);
   ctx->release(ctx->wf_ctl);
   ctx->trim(0);
   if (ctx->h_live) cudaFreeHost(ctx->h_live);
@@ -1338,8 +1339,22 @@ int vt::render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32
     ctx->launches += (uint64_t)passes[i];
   }
   if (wf_jobs.empty()) return VT_OK;
+  // counted passes and calls that set the wavefront's shape keep the wavefront
+  const bool by_size = kernel == 0 && path_slots <= 0 && blocks_per_sm <= 0 && !count;
   return render_wavefront(ctx, wf_jobs.data(), (int32_t)wf_jobs.size(), wf_passes.data(), path_slots, blocks_per_sm,
-                          count);
+                          count, by_size);
+}
+
+// Sample buffer of a launch.
+static int sbuf_reserve(vt_context* ctx, int64_t items) {
+  if (ctx->sbuf_items >= items) return VT_OK;
+  ctx->release(ctx->sbuf);
+  ctx->sbuf = nullptr;
+  ctx->sbuf_items = 0;
+  int rc = ctx->alloc((void**)&ctx->sbuf, sizeof(float4) * (size_t)items);
+  if (rc != VT_OK) return rc;
+  ctx->sbuf_items = items;
+  return VT_OK;
 }
 
 // Device buffers of the wavefront for `slots` path slots and `items` samples.
@@ -1353,13 +1368,9 @@ static int wf_reserve(vt_context* ctx, int64_t slots, int64_t items) {
     if (rc != VT_OK) return rc;
     ctx->wf_slots = slots;
   }
-  if (ctx->sbuf_items < items) {
-    ctx->release(ctx->sbuf);
-    ctx->sbuf = nullptr;
-    ctx->sbuf_items = 0;
-    int rc = ctx->alloc((void**)&ctx->sbuf, sizeof(float4) * (size_t)items);
+  {
+    int rc = sbuf_reserve(ctx, items);
     if (rc != VT_OK) return rc;
-    ctx->sbuf_items = items;
   }
   if (!ctx->wf_ctl) {
     int rc = ctx->alloc((void**)&ctx->wf_ctl, vt_context::kMaxLanes * kCtlBytes);
@@ -1380,22 +1391,64 @@ static int wf_reserve(vt_context* ctx, int64_t slots, int64_t items) {
   return VT_OK;
 }
 
-// One wavefront launch over `entries` (tile_begin = first item of each job).
-static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std::vector<Grid>& grids,
-                     int64_t items, int64_t slots_cap, int blocks_per_sm, bool count) {
-  vt::Range nvtx_range("vt.wavefront_launch");
-  const int64_t slots = std::max<int64_t>(32, std::min<int64_t>(items, slots_cap));
-  int rc = wf_reserve(ctx, slots, items);
-  if (rc != VT_OK) return rc;
+// Device copy of a launch's job records.
+static int jobs_upload(vt_context* ctx, const std::vector<JobEntry>& entries) {
   const size_t jbytes = sizeof(JobEntry) * entries.size();
   if (ctx->d_jobs_bytes < jbytes) {
     ctx->release(ctx->d_jobs);
     ctx->d_jobs = nullptr;
     ctx->d_jobs_bytes = 0;
-    rc = ctx->alloc((void**)&ctx->d_jobs, jbytes);
+    int rc = ctx->alloc((void**)&ctx->d_jobs, jbytes);
     if (rc != VT_OK) return rc;
     ctx->d_jobs_bytes = jbytes;
   }
+  VT_CUDA(cudaMemcpyAsync(ctx->d_jobs, entries.data(), jbytes, cudaMemcpyHostToDevice, ctx->stream), "job table");
+  return VT_OK;
+}
+
+// Samples per launch up to which each gets a thread of its own (k_paths), and
+// up to which block wavefronts carry them (k_paths_block, with the times on
+// both sides of either line).
+constexpr int64_t kPathsItems = 1 << 17;
+constexpr int64_t kBlockItems = 3 << 20;
+
+// A launch of at most kPathsItems samples: one kernel over the samples, then
+// the accumulation; a single pass of one job accumulates as it goes.
+static int paths_launch(vt_context* ctx, const std::vector<JobEntry>& entries, int64_t items) {
+  if (entries.size() == 1 && entries[0].passes == 1) {
+    VT_CUDA(launch_plain(entries[0].F, entries[0].J, entries[0].sample_base, 1, nullptr, ctx->stream), "pass");
+    ctx->launches += 1;
+    return VT_OK;
+  }
+  int rc = sbuf_reserve(ctx, items);
+  if (rc == VT_OK) rc = jobs_upload(ctx, entries);
+  if (rc != VT_OK) return rc;
+  WfJobTable table;
+  if (entries.size() <= (size_t)kWfParamJobs) {
+    memset(&table, 0, sizeof(table));
+    for (size_t i = 0; i < entries.size(); ++i) table.e[i] = entries[i];
+  }
+  WfParams P;
+  memset(&P, 0, sizeof(P));
+  P.jobs = ctx->d_jobs;
+  P.n_jobs = (int32_t)entries.size();
+  P.n_items = (unsigned long long)items;
+  P.sbuf = ctx->sbuf;
+  VT_CUDA(launch_paths(P, ctx->stream, entries.size() <= (size_t)kWfParamJobs ? &table : nullptr), "samples");
+  long long max_pixels = 0;
+  for (const JobEntry& e : entries) max_pixels = std::max<long long>(max_pixels, e.n_pixels);
+  VT_CUDA(launch_wf_accumulate(ctx->d_jobs, (int)entries.size(), max_pixels, ctx->sbuf, ctx->stream), "accumulate");
+  ctx->launches += 2;
+  return VT_OK;
+}
+
+// A launch as block wavefronts: every block carries its own paths from camera
+// to sample buffer, so one kernel takes the whole launch.
+static int block_launch(vt_context* ctx, const std::vector<JobEntry>& entries, const std::vector<Grid>& grids,
+                        int64_t items) {
+  int rc = sbuf_reserve(ctx, items);
+  if (rc == VT_OK) rc = jobs_upload(ctx, entries);
+  if (rc != VT_OK) return rc;
   const size_t gbytes = sizeof(Grid) * grids.size();
   if (ctx->d_grids_bytes < gbytes) {
     ctx->release(ctx->d_grids);
@@ -1406,7 +1459,84 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
     ctx->d_grids_bytes = gbytes;
   }
   cudaStream_t st = ctx->stream;
-  VT_CUDA(cudaMemcpyAsync(ctx->d_jobs, entries.data(), jbytes, cudaMemcpyHostToDevice, st), "job table");
+  VT_CUDA(cudaMemcpyAsync(ctx->d_grids, grids.data(), gbytes, cudaMemcpyHostToDevice, st), "grid table");
+  // a third of a block's share of the samples in flight, the block's threads at least
+  const int blocks = (int)std::min<int64_t>((int64_t)ctx->sm_count * kBlocksPerSm, (items + 31) / 32);
+  const int64_t share = (items + blocks - 1) / blocks;
+  const int64_t want = std::min<int64_t>(share, std::max<int64_t>((share + 2) / 3, kBlockThreads));
+  const int slots = (int)std::min<int64_t>((want + 31) / 32 * 32, kBlockSlots);
+  const size_t bytes = (size_t)blocks * kBlockFields * slots * sizeof(float4);
+  if (ctx->block_bytes < bytes) {
+    ctx->release(ctx->block_state);
+    ctx->block_state = nullptr;
+    ctx->block_bytes = 0;
+    rc = ctx->alloc((void**)&ctx->block_state, bytes);
+    if (rc != VT_OK) return rc;
+    ctx->block_bytes = bytes;
+  }
+  WfJobTable table;
+  const WfJobTable* T = nullptr;
+  BlockParams P;
+  memset(&P, 0, sizeof(P));
+  P.bricks_444 = 1;
+  for (const Grid& g : grids)
+    if (g.shx != 2 || g.shy != 2 || g.shz != 2) P.bricks_444 = 0;
+  if (entries.size() <= (size_t)kWfParamJobs) {
+    memset(&table, 0, sizeof(table));
+    for (size_t i = 0; i < entries.size(); ++i) {
+      table.e[i] = entries[i];
+      table.g[i] = grids[i];
+    }
+    T = &table;
+  }
+  int32_t max_b = 0;
+  for (const JobEntry& e : entries) max_b = std::max(max_b, e.F.max_bounces);
+  P.jobs = ctx->d_jobs;
+  P.n_jobs = (int32_t)entries.size();
+  P.slots = slots;
+  P.grids = ctx->d_grids;
+  P.state = ctx->block_state;
+  P.next_item = ctx->d_queue + 2;
+  P.n_items = (unsigned long long)items;
+  P.sbuf = ctx->sbuf;
+  P.trace_steps = ctx->trace_steps;
+  // a path ends within max_bounces + 2 rounds of its start: the wavefront's
+  // bound, for a block that takes every sample
+  P.max_rounds = (int32_t)std::min<int64_t>(4 * (items / slots + 2) * ((int64_t)max_b + 2) + 16, 0x7fffffff);
+  P.error = ctx->d_error;
+  VT_CUDA(cudaMemsetAsync(P.next_item, 0, sizeof(unsigned long long), st), "block wavefront");
+  VT_CUDA(cudaMemsetAsync(P.error, 0, sizeof(int32_t), st), "block wavefront");
+  VT_CUDA(launch_paths_block(P, blocks, st, T), "block wavefront");
+  long long max_pixels = 0;
+  for (const JobEntry& e : entries) max_pixels = std::max<long long>(max_pixels, e.n_pixels);
+  VT_CUDA(launch_wf_accumulate(ctx->d_jobs, (int)entries.size(), max_pixels, ctx->sbuf, st), "accumulate");
+  ctx->launches += 2;
+  int32_t error = 0;   // pageable: the read has completed when the copy returns
+  VT_CUDA(cudaMemcpyAsync(&error, P.error, sizeof(error), cudaMemcpyDeviceToHost, st), "block wavefront");
+  VT_CUDA(cudaStreamSynchronize(st), "block wavefront");
+  if (error) return fail(VT_EDEVICE, "wavefront did not drain within %d rounds of a block", P.max_rounds);
+  return VT_OK;
+}
+
+// One wavefront launch over `entries` (tile_begin = first item of each job).
+static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std::vector<Grid>& grids,
+                     int64_t items, int64_t slots_cap, int blocks_per_sm, bool count) {
+  vt::Range nvtx_range("vt.wavefront_launch");
+  const int64_t slots = std::max<int64_t>(32, std::min<int64_t>(items, slots_cap));
+  int rc = wf_reserve(ctx, slots, items);
+  if (rc != VT_OK) return rc;
+  rc = jobs_upload(ctx, entries);
+  if (rc != VT_OK) return rc;
+  const size_t gbytes = sizeof(Grid) * grids.size();
+  if (ctx->d_grids_bytes < gbytes) {
+    ctx->release(ctx->d_grids);
+    ctx->d_grids = nullptr;
+    ctx->d_grids_bytes = 0;
+    rc = ctx->alloc((void**)&ctx->d_grids, gbytes);
+    if (rc != VT_OK) return rc;
+    ctx->d_grids_bytes = gbytes;
+  }
+  cudaStream_t st = ctx->stream;
   VT_CUDA(cudaMemcpyAsync(ctx->d_grids, grids.data(), gbytes, cudaMemcpyHostToDevice, st), "grid table");
   WfJobTable table;
   const WfJobTable* T = nullptr;
@@ -1553,11 +1683,11 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
 // Wavefront rendering of passes[i] samples per pixel for each job, split in
 // launches whose sample buffers stay within ctx->max_items.
 int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32_t* passes, int slots,
-                         int blocks_per_sm, bool count) {
+                         int blocks_per_sm, bool count, bool by_size) {
   if (n > kWfMaxJobs) {   // launches of at most kWfMaxJobs jobs
     for (int32_t i = 0; i < n; i += kWfMaxJobs) {
       const int rc = render_wavefront(ctx, jobs + i, std::min<int32_t>(kWfMaxJobs, n - i), passes + i, slots,
-                                      blocks_per_sm, count);
+                                      blocks_per_sm, count, by_size);
       if (rc != VT_OK) return rc;
     }
     return VT_OK;
@@ -1590,7 +1720,9 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
       done[i] += p;
     }
     if (items >= ((int64_t)1 << 32)) return fail(VT_EINVAL, "more than 2^32 samples in one launch");
-    int rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
+    int rc = by_size && items <= kPathsItems   ? paths_launch(ctx, entries, items)
+             : by_size && items <= kBlockItems ? block_launch(ctx, entries, grids, items)
+                                             : wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
     if (rc != VT_OK) return rc;
   }
   return VT_OK;

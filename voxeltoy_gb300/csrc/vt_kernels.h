@@ -112,6 +112,30 @@ cudaError_t launch_wf_shade(const WfParams& P, int par, int persist_blocks, bool
                             const WfJobTable* T = nullptr);
 cudaError_t launch_wf_trace(const WfParams& P, int par, int blocks, int steps, bool count, cudaStream_t st,
                             const WfJobTable* T = nullptr);
+// Block wavefront (k_paths_block): `blocks` blocks, each with the state of
+// `slots` paths (kBlockFields float4 arrays of that many entries).
+constexpr int kBlockThreads = 256;
+constexpr int kBlocksPerSm = 4;
+constexpr int kBlockSlots = 1024;      // most slots a block can hold
+constexpr int kBlockFields = 9;
+struct BlockParams {
+  const JobEntry* jobs;            // device array, tile_begin = first item of the job
+  int32_t n_jobs;
+  int32_t slots;                   // paths in flight per block, at most kBlockSlots
+  const Grid* grids;
+  float4* state;                   // blocks * kBlockFields * slots
+  unsigned long long* next_item;   // zero before the launch
+  unsigned long long n_items;
+  float4* sbuf;                    // per-item sample outputs
+  int32_t bricks_444;              // every job's bricks are 4x4x4
+  int32_t trace_steps;             // DDA steps between refills (a multiple of 4)
+  int32_t max_rounds;              // bound of a block's loop
+  int32_t* error;                  // set if a block reaches it
+};
+cudaError_t launch_paths_block(const BlockParams& P, int blocks, cudaStream_t st, const WfJobTable* T = nullptr);
+// Every sample of a launch by a thread of its own (jobs, n_jobs, n_items and
+// sbuf of P), outputs into sbuf as the wavefront's.
+cudaError_t launch_paths(const WfParams& P, cudaStream_t st, const WfJobTable* T = nullptr);
 cudaError_t launch_wf_accumulate(const JobEntry* jobs, int n_jobs, long long max_pixels, const float4* sbuf,
                                  cudaStream_t st);
 int wf_trace_blocks_per_sm();

@@ -9,6 +9,9 @@
 //                 (DDA of every queued segment with per-warp refill from the
 //                 queue); per-sample outputs land in a sample buffer that
 //                 k_wf_accumulate reduces in sample order.
+//   k_paths       one thread per sample (launches of few samples)
+//   k_paths_block wavefronts inside blocks, one kernel per launch (launches of
+//                 up to a few million samples)
 //   k_diag        per-sample output and first-hit record (parity tests)
 //   k_trace_rays  DDA of caller-supplied rays (parity tests)
 //   k_pick        focal-distance pick of one pixel (focalDistance.vs:45-81)
@@ -109,25 +112,32 @@ __device__ __forceinline__ float4 pack4(v3 a, float w) { return make_float4(a.x,
 struct WfNoTable {
   int unused;
 };
-__device__ __forceinline__ const JobEntry& job_entry(const WfParams& P, const WfNoTable&, uint32_t j) {
+template <class Par>
+__device__ __forceinline__ const JobEntry& job_entry(const Par& P, const WfNoTable&, uint32_t j) {
   return P.jobs[j];
 }
-__device__ __forceinline__ const JobEntry& job_entry(const WfParams&, const WfJobTable& T, uint32_t j) {
+template <class Par>
+__device__ __forceinline__ const JobEntry& job_entry(const Par&, const WfJobTable& T, uint32_t j) {
   return T.e[j];
 }
-__device__ __forceinline__ const Grid& grid_entry(const WfParams& P, const WfNoTable&, uint32_t j) {
+template <class Par>
+__device__ __forceinline__ const Grid& grid_entry(const Par& P, const WfNoTable&, uint32_t j) {
   return P.grids[j];
 }
-__device__ __forceinline__ const Grid& grid_entry(const WfParams&, const WfJobTable& T, uint32_t j) {
+template <class Par>
+__device__ __forceinline__ const Grid& grid_entry(const Par&, const WfJobTable& T, uint32_t j) {
   return T.g[j];
 }
-__device__ __forceinline__ const JobEntry& job_entry(const WfParams&, const WfOneJob& T, uint32_t) { return T.e; }
-__device__ __forceinline__ const Grid& grid_entry(const WfParams&, const WfOneJob& T, uint32_t) { return T.g; }
+template <class Par>
+__device__ __forceinline__ const JobEntry& job_entry(const Par&, const WfOneJob& T, uint32_t) { return T.e; }
+template <class Par>
+__device__ __forceinline__ const Grid& grid_entry(const Par&, const WfOneJob& T, uint32_t) { return T.g; }
 
 // Job of a global item index (binary search over tile_begin).
-__device__ __forceinline__ int job_of(const WfParams&, const WfOneJob&, unsigned long long) { return 0; }
-template <class Tab>
-__device__ __forceinline__ int job_of(const WfParams& P, const Tab& T, unsigned long long item) {
+template <class Par>
+__device__ __forceinline__ int job_of(const Par&, const WfOneJob&, unsigned long long) { return 0; }
+template <class Par, class Tab>
+__device__ __forceinline__ int job_of(const Par& P, const Tab& T, unsigned long long item) {
   int lo = 0, hi = P.n_jobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
@@ -487,12 +497,14 @@ __global__ void __launch_bounds__(128, RegenBlocks<Tab>::value) k_wf_regen(const
 template <class Tab>
 struct GridHold {
   Grid g;
-  __device__ __forceinline__ void set(const WfParams& P, const Tab& T, uint32_t job) { g = grid_entry(P, T, job); }
+  template <class Par>
+  __device__ __forceinline__ void set(const Par& P, const Tab& T, uint32_t job) { g = grid_entry(P, T, job); }
   __device__ __forceinline__ const Grid& get(const Tab&) const { return g; }
 };
 template <>
 struct GridHold<WfOneJob> {
-  __device__ __forceinline__ void set(const WfParams&, const WfOneJob&, uint32_t) {}
+  template <class Par>
+  __device__ __forceinline__ void set(const Par&, const WfOneJob&, uint32_t) {}
   __device__ __forceinline__ const Grid& get(const WfOneJob& T) const { return T.g; }
 };
 
@@ -686,6 +698,295 @@ __global__ void __launch_bounds__(256, 4) k_wf_trace_pool(const WfParams P, cons
   flush_counters(cnt, P.counters);
 }
 
+// ------------------------------------------------------- block wavefront
+// The wavefront's round in one block: each block holds `slots` paths (their
+// state in a region of its own, L2-resident; lists of slots and of segments in
+// shared memory) and takes them through rounds of the same four parts, with
+// block barriers where the wavefront starts a kernel, drawing new samples from
+// one counter until none is left.  Blocks never wait for one another, so a
+// launch is one kernel.
+//
+// A wavefront launch costs some 0.45 ms before its first path (0.85 ms with
+// eight bounces: two groups of rounds): kernels of a few microseconds, five a
+// round and lane, and the capture of their graph.  Here a round costs its
+// block three barriers.  Per sample the block form is the slower one: all
+// four parts run at the registers of the largest (64, 1024 threads an SM), and
+// a block of a thousand paths ends every DDA part waiting for its longest
+// segments.  Measured (us, thread per sample / block / wavefront):
+//   19 k samples of 64^3 spheres          142 /  170 /  435
+//   262 k of 128^3 noise, 8 bounces       610 /  460 /  975
+//   1.05 M of 64^3 spheres                805 /  561 /  744
+//   2.1 M of a 203x117x89 noise volume   1477 /  688 /  928
+//   3.1 M of 128^3 noise, 256^3 noise       - / 2219, 2916 / 2272, 3025
+//   3.1 M of a 1024^3 shell                 - / 6230 / 5817
+//   4.2 M of 128^3 noise                    - / 2930 / 2672
+//   8.6 M of a 203x117x89 noise volume      - / 2042 / 1950
+// 512 slots against 1024: 545 and 568 us at 1.05 M samples, 748 and 676 at
+// 2.1 M: about a third of a block's samples in flight is best.
+// State fields of a path slot.
+enum {
+  BF_RO = 0,       // ro.xyz, -
+  BF_RD = 1,       // rd.xyz, item
+  BF_L = 2,        // L.xyz, rng word
+  BF_T = 3,        // T.xyz, bsdf_pdf
+  BF_NEE = 4,      // nee_P.xyz, light
+  BF_EXT = 5,      // extension segment: vo.xyz, inc.x; next field: inc.yz, end (8 bytes)
+  BF_SHADOW = 7,   // shadow segment, the same
+};
+enum { BC_LAMBERT = 0, BC_OTHER = 1, BC_FREE = 2, BC_QUEUE = 3, BC_HEAD = 4, BC_NUM = 5 };
+
+// Entry of this lane in a shared list after `ctr` for the lanes with `want`:
+// one shared atomic per warp.  All lanes of the warp must call it.
+__device__ __forceinline__ uint32_t warp_push(uint32_t* ctr, bool want, int lane, unsigned lt) {
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  uint32_t base = 0;
+  if (lane == 0 && m) base = atomicAdd(ctr, (uint32_t)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  return base + __popc(m & lt);
+}
+
+template <bool k444, class Tab>
+__global__ void __launch_bounds__(kBlockThreads, kBlocksPerSm) k_paths_block(const BlockParams P,
+                                                                            const __grid_constant__ Tab T) {
+  __shared__ uint32_t s_flags[kBlockSlots];
+  __shared__ uint16_t s_queue[2 * kBlockSlots];
+  __shared__ uint16_t s_hits[kBlockSlots];
+  __shared__ uint16_t s_free[kBlockSlots];
+  __shared__ uint32_t s_n[2][BC_NUM];
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int warp_first = threadIdx.x & ~31;
+  const int S = P.slots;
+  float4* const st = P.state + (size_t)blockIdx.x * kBlockFields * S;
+  Cnt<false> cnt;
+  for (int i = threadIdx.x; i < S; i += kBlockThreads) s_flags[i] = 0u;
+  if (threadIdx.x < 2 * BC_NUM) s_n[threadIdx.x / BC_NUM][threadIdx.x % BC_NUM] = 0u;
+  __syncthreads();
+  for (int round = 0;; ++round) {
+    if (round >= P.max_rounds) {
+      if (threadIdx.x == 0) *P.error = 1;
+      break;
+    }
+    uint32_t* const ctr = s_n[round & 1];
+    // ---- segment ends: finished paths out, kept hits and free slots listed
+    for (int b0 = warp_first; b0 < S; b0 += kBlockThreads) {
+      const int i = b0 + lane;
+      const bool mine = i < S;
+      const uint32_t fl = mine ? s_flags[i] : 0u;
+      bool hit = false;
+      int cls = 0;
+      if (fl & SL_ACTIVE) {
+        const JobEntry& E = job_entry(P, T, fl >> kSlotJobShift);
+        Path p;
+        // every load of the slot is issued before any of them is used
+        const float4 a1 = st[BF_RD * S + i], a3 = st[BF_L * S + i], a4 = st[BF_T * S + i];
+        float4 a5 = make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned long long hs = 0ull, he = 0ull;
+        if (fl & SL_SHADOW) {
+          a5 = st[BF_NEE * S + i];
+          hs = ((const unsigned long long*)&st[(BF_SHADOW + 1) * S + i])[1];
+        }
+        if (fl & SL_EXT) he = ((const unsigned long long*)&st[(BF_EXT + 1) * S + i])[1];
+        p.rd = xyz4(a1);
+        const uint32_t item = __float_as_uint(a1.w);
+        p.L = xyz4(a3);
+        p.T = xyz4(a4); p.bsdf_pdf = a4.w;
+        p.nee_P = xyz4(a5); p.light = __float_as_int(a5.w);
+        load_flags(fl, p);
+        if (fl & SL_SHADOW) shadow_end(E.F, p, unpack_end(hs));
+        if (fl & SL_EXT) {
+          const SegEnd e = unpack_end(he);
+          hit = ext_resolve(E.F, E.J, p, e, cnt);
+          if (hit) cls = hit_class(E.F, E.J, e);
+        }
+        if (hit) {
+          if (fl & SL_SHADOW) st[BF_L * S + i] = pack4(p.L, a3.w);
+          s_flags[i] = slot_flags(p, 1u, fl >> kSlotJobShift);
+        } else {
+          if (chk(item < P.n_items, CHK_SAMPLE)) P.sbuf[item] = path_output(E.F, p);
+          s_flags[i] = 0u;
+        }
+      }
+      const uint32_t jl = warp_push(&ctr[BC_LAMBERT], hit && cls == 0, lane, lt);
+      const uint32_t jo = warp_push(&ctr[BC_OTHER], hit && cls != 0, lane, lt);
+      const uint32_t jf = warp_push(&ctr[BC_FREE], mine && !hit, lane, lt);
+      if (hit) s_hits[cls == 0 ? jl : (uint32_t)S - 1u - jo] = (uint16_t)i;
+      else if (mine) s_free[jf] = (uint16_t)i;
+    }
+    if (threadIdx.x < BC_NUM) s_n[(round & 1) ^ 1][threadIdx.x] = 0u;   // the next round's counters
+    __syncthreads();
+    // ---- vertices of the kept hits, Lambert first
+    const uint32_t nl = ctr[BC_LAMBERT], n_hits = nl + ctr[BC_OTHER], n_free = ctr[BC_FREE];
+    for (uint32_t v0 = warp_first; v0 < n_hits; v0 += kBlockThreads) {
+      const uint32_t v = v0 + lane;
+      const bool mine = v < n_hits;
+      uint32_t emit = 0u, i = 0u;
+      if (mine) {
+        i = s_hits[v < nl ? v : (uint32_t)S - 1u - (v - nl)];
+        const uint32_t fl = s_flags[i];
+        const float4 h0 = st[BF_RO * S + i], h1 = st[BF_RD * S + i], h2 = st[BF_L * S + i], h3 = st[BF_T * S + i];
+        const unsigned long long he = ((const unsigned long long*)&st[(BF_EXT + 1) * S + i])[1];
+        const uint32_t job = fl >> kSlotJobShift;
+        const JobEntry& E = job_entry(P, T, job);
+        Path p;
+        p.ro = xyz4(h0);
+        p.rd = xyz4(h1);
+        const uint32_t item = __float_as_uint(h1.w);
+        p.L = xyz4(h2);
+        p.T = xyz4(h3); p.bsdf_pdf = h3.w;
+        load_flags(fl, p);
+        rng_from_item(E, item, __float_as_uint(h2.w), p);
+        ext_hit(E.F, E.J, p, unpack_end(he), cnt);
+        emit = 2u | (p.has_cont ? 1u : 0u);
+        const uint32_t rng = (E.F.rng_mode == 1) ? ((uint32_t)p.rng.ox | ((uint32_t)p.rng.oy << 16)) : p.rng.call;
+        st[BF_RO * S + i] = pack4(p.ro, 0.0f);
+        st[BF_RD * S + i] = pack4(p.rd, __uint_as_float(item));
+        st[BF_L * S + i] = pack4(p.L, __uint_as_float(rng));
+        st[BF_T * S + i] = pack4(p.T, p.bsdf_pdf);
+        st[BF_NEE * S + i] = pack4(p.nee_P, __int_as_float(p.light));
+        if (emit & 1u) {
+          const SegRec sr = seg_rec(E.F, p.ro, p.rd);
+          st[BF_EXT * S + i] = make_float4(sr.vo.x, sr.vo.y, sr.vo.z, sr.inc.x);
+          *(float2*)&st[(BF_EXT + 1) * S + i] = make_float2(sr.inc.y, sr.inc.z);
+        }
+        const SegRec sr = seg_rec(E.F, p.ro, p.sd);
+        st[BF_SHADOW * S + i] = make_float4(sr.vo.x, sr.vo.y, sr.vo.z, sr.inc.x);
+        *(float2*)&st[(BF_SHADOW + 1) * S + i] = make_float2(sr.inc.y, sr.inc.z);
+        s_flags[i] = slot_flags(p, emit, job);
+      }
+      const uint32_t q1 = warp_push(&ctr[BC_QUEUE], (emit & 1u) != 0u, lane, lt);
+      if (emit & 1u) s_queue[q1] = (uint16_t)(i << 1);
+      const uint32_t q2 = warp_push(&ctr[BC_QUEUE], (emit & 2u) != 0u, lane, lt);
+      if (emit & 2u) s_queue[q2] = (uint16_t)((i << 1) | 1u);
+    }
+    // ---- new paths in the free slots
+    for (uint32_t k0 = warp_first; k0 < n_free; k0 += kBlockThreads) {
+      const bool left = lane == 0 && *(volatile unsigned long long*)P.next_item < P.n_items;
+      if (!__any_sync(FULL, left)) break;
+      const uint32_t k = k0 + lane;
+      const bool mine = k < n_free;
+      bool need_new = mine, active = false;
+      Path p;
+      uint32_t job = 0, item = 0;
+      float t_enter = 0.0f;
+      for (;;) {
+        const unsigned want = __ballot_sync(FULL, need_new);
+        if (!want) break;
+        unsigned long long my = 0;
+        if (lane == 0) my = atomicAdd(P.next_item, (unsigned long long)__popc(want));
+        my = __shfl_sync(FULL, my, 0) + __popc(want & lt);
+        if (!need_new) continue;
+        if (my >= P.n_items) {
+          need_new = false;   // no items left
+        } else {
+          item = (uint32_t)my;
+          job = (uint32_t)job_of(P, T, my);
+          const JobEntry& E = job_entry(P, T, job);
+          const uint32_t r = (uint32_t)(my - (unsigned long long)E.tile_begin);   // < 2^32 items per launch
+          const uint32_t pass = udiv(r, E.F.m_pixels);
+          const uint32_t pixel = r - pass * (uint32_t)E.n_pixels;
+          const uint32_t py = udiv(pixel, E.F.m_width), px = pixel - py * (uint32_t)E.F.width;
+          if (path_start(E.F, E.J, p, (int)px, (int)py, E.sample_base + (int)pass, cnt, t_enter)) {
+            active = true;
+            need_new = false;
+          } else if (chk(item < P.n_items, CHK_SAMPLE)) {
+            P.sbuf[item] = path_output(E.F, p);   // missed the volume: finished, take another item
+          }
+        }
+      }
+      const uint32_t q1 = warp_push(&ctr[BC_QUEUE], active, lane, lt);
+      if (active) {
+        const uint32_t i = s_free[k];
+        const Frame& F = job_entry(P, T, job).F;
+        const uint32_t rng = (F.rng_mode == 1) ? ((uint32_t)p.rng.ox | ((uint32_t)p.rng.oy << 16)) : p.rng.call;
+        const v3 o = p.ro + t_enter * p.rd;   // the primary segment starts at the volume entry point
+        const SegRec sr = seg_rec(F, o, p.rd);
+        st[BF_RO * S + i] = pack4(p.ro, 0.0f);
+        st[BF_RD * S + i] = pack4(p.rd, __uint_as_float(item));
+        st[BF_L * S + i] = pack4(p.L, __uint_as_float(rng));
+        st[BF_T * S + i] = pack4(p.T, p.bsdf_pdf);
+        st[BF_EXT * S + i] = make_float4(sr.vo.x, sr.vo.y, sr.vo.z, sr.inc.x);
+        *(float2*)&st[(BF_EXT + 1) * S + i] = make_float2(sr.inc.y, sr.inc.z);
+        s_flags[i] = slot_flags(p, 1u, job);
+        s_queue[q1] = (uint16_t)(i << 1);
+      }
+    }
+    __syncthreads();
+    // ---- DDA of every listed segment
+    const uint32_t n = ctr[BC_QUEUE];
+    if (n == 0u) break;   // no path is left, and no item was
+    {
+      bool have = false, more = true;
+      GridHold<Tab> gh;
+      Dda s;
+      uint32_t tag = 0u;
+      for (;;) {
+        const unsigned need = __ballot_sync(FULL, !have);
+        if (need && more) {
+          const uint32_t want = __popc(need);
+          uint32_t c = 0;
+          if (lane == 0) c = atomicAdd(&ctr[BC_HEAD], want);
+          c = __shfl_sync(FULL, c, 0);
+          more = c + want < n;
+          const uint32_t rec = c + __popc(need & lt);
+          if (!have && rec < n) {
+            tag = s_queue[rec];
+            const float4* at = st + (BF_EXT + 2 * (tag & 1u)) * S + (tag >> 1);
+            const float4 na = at[0];
+            const float2 nb = *(const float2*)&at[S];
+            gh.set(P, T, s_flags[tag >> 1] >> kSlotJobShift);
+            dda_begin_rec(gh.get(T), s, mk3(na.x, na.y, na.z), mk3(na.w, nb.x, nb.y));
+            if (k444 && s.state == DDA_RUNNING) dda_end_stuck(gh.get(T), s);
+            if (s.state == DDA_RUNNING) have = true;
+            else ((unsigned long long*)&st[(BF_EXT + 1 + 2 * (tag & 1u)) * S + (tag >> 1)])[1] =
+                     pack_end(s.x, s.y, s.z, s.state);
+          }
+        }
+        if (!more && !__any_sync(FULL, have)) break;
+        if (have) {
+          if constexpr (k444) dda_steps_444<false>(gh.get(T), s, P.trace_steps, 0);
+          else dda_steps<false, false, false>(gh.get(T), s, P.trace_steps, cnt, 0);
+          if (s.state != DDA_RUNNING) {
+            ((unsigned long long*)&st[(BF_EXT + 1 + 2 * (tag & 1u)) * S + (tag >> 1)])[1] =
+                pack_end_inside(s.x, s.y, s.z, s.state);
+            have = false;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <class Tab>
+static void paths_block(const BlockParams& P, const Tab& T, int blocks, cudaStream_t st) {
+  if (P.bricks_444) k_paths_block<true><<<blocks, kBlockThreads, 0, st>>>(P, T);
+  else k_paths_block<false><<<blocks, kBlockThreads, 0, st>>>(P, T);
+}
+static WfOneJob one_job(const WfJobTable& T);
+cudaError_t launch_paths_block(const BlockParams& P, int blocks, cudaStream_t st, const WfJobTable* T) {
+  if (T && P.n_jobs == 1) paths_block(P, one_job(*T), blocks, st);
+  else if (T && P.n_jobs <= kWfParamJobs) paths_block(P, *T, blocks, st);
+  else paths_block(P, WfNoTable{0}, blocks, st);
+  return cudaGetLastError();
+}
+
+// Launches of few samples, where only the longest path's time counts: one
+// thread carries a whole sample from the camera to its output.
+template <class Tab>
+__global__ void __launch_bounds__(128) k_paths(const WfParams P, const __grid_constant__ Tab T) {
+  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= P.n_items) return;
+  const JobEntry& E = job_entry(P, T, (uint32_t)job_of(P, T, i));
+  const uint32_t r = (uint32_t)(i - (unsigned long long)E.tile_begin);
+  const uint32_t pass = udiv(r, E.F.m_pixels);
+  const uint32_t pixel = r - pass * (uint32_t)E.n_pixels;
+  const uint32_t py = udiv(pixel, E.F.m_width), px = pixel - py * (uint32_t)E.F.width;
+  Cnt<false> cnt;
+  P.sbuf[i] = trace_sample(E.F, E.J, (int)px, (int)py, E.sample_base + (int)pass, cnt, (HitRecord*)nullptr);
+}
+
 // Ordered reduction of the per-sample outputs into each pixel's Kahan sums:
 // sample order within a pixel is the same as one sample per launch.
 __global__ void k_wf_accumulate(const JobEntry* jobs, const float4* sbuf) {
@@ -724,6 +1025,14 @@ cudaError_t launch_wf_shade(const WfParams& P, int par, int persist_blocks, bool
   if (T && P.n_jobs == 1) wf_shade(P, one_job(*T), par, persist_blocks, count, st);
   else if (T && P.n_jobs <= kWfParamJobs) wf_shade(P, *T, par, persist_blocks, count, st);
   else wf_shade(P, WfNoTable{0}, par, persist_blocks, count, st);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_paths(const WfParams& P, cudaStream_t st, const WfJobTable* T) {
+  const unsigned blocks = (unsigned)((P.n_items + 127) / 128);
+  if (T && P.n_jobs == 1) k_paths<<<blocks, 128, 0, st>>>(P, one_job(*T));
+  else if (T && P.n_jobs <= kWfParamJobs) k_paths<<<blocks, 128, 0, st>>>(P, *T);
+  else k_paths<<<blocks, 128, 0, st>>>(P, WfNoTable{0});
   return cudaGetLastError();
 }
 
@@ -809,7 +1118,10 @@ __global__ void k_trace_rays(const Frame F, const JobDev J, const float* origins
   Dda s;
   const Grid g = grid_of(F, J);
   dda_begin(g, s, o, d);
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  if (s.state == DDA_RUNNING) {   // the loops that count steps
+    if (bricks_444(g)) dda_steps<false, false, true>(g, s, 0x7fffffff, cnt, 0);
+    else dda_steps<false, false, false>(g, s, 0x7fffffff, cnt, 0);
+  }
   const bool h = dda_hit(F, s);
   int flags = (h ? 1 : 0) << 8 | ((h && s.state != DDA_HIT) ? 1 : 0) << 9 | (s.steps << 10);
   if (h) {
@@ -844,7 +1156,7 @@ __global__ void k_pick(const Frame F, const JobDev J, float x, float y, float* o
   Dda s;
   const Grid g = grid_of(F, J);
   dda_begin(g, s, o + t * d, d);
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  dda_finish(g, s, cnt);
   if (!dda_hit(F, s)) return;
   const v3 vs = ld3(F.vsize);
   const v3 vmin = mk3((float)s.x, (float)s.y, (float)s.z) * vs + ld3(F.bmin);
@@ -871,7 +1183,7 @@ __global__ void k_select(const Frame F, const JobDev J, float x, float y, float 
   Dda s;
   const Grid g = grid_of(F, J);
   dda_begin(g, s, o + t * d, d);
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  dda_finish(g, s, cnt);
   if (!dda_hit(F, s)) return;
   const Basis b = voxel_basis(F, s.x, s.y, s.z, o, d);
   out[0] = s.x; out[1] = s.y; out[2] = s.z; out[3] = 1;

@@ -19,7 +19,7 @@ struct vt_context {
   uint64_t budget = 0;          // 0 = unlimited
   uint64_t in_use = 0;          // bytes held through alloc()
   int sm_count = 0;
-  int kernel = 2;               // 1 plain, 2 wavefront
+  int kernel = 0;               // 0 by the launch's size, 1 plain, 2 wavefront
   vt_log_fn log_fn = nullptr;
   void* log_user = nullptr;
   std::mutex mu;
@@ -34,6 +34,8 @@ struct vt_context {
   size_t d_grids_bytes = 0;
   void* wf_mem = nullptr;        // slot state, flags, hits, queues
   int64_t wf_slots = 0;
+  float4* block_state = nullptr; // path state of the block wavefront
+  size_t block_bytes = 0;
   float4* sbuf = nullptr;        // per-sample outputs of one launch
   int64_t sbuf_items = 0;
   uint32_t* wf_ctl = nullptr;    // control words, one kCtlBytes block per lane (layout of ctl_index)
@@ -149,10 +151,12 @@ void release_context(vt_context* ctx);
 int fixed_scratch_setup(int device);
 // Rebuilds a job's frame when its scene was edited since (scene->generation).
 int refresh_job(vt_job* j);
-// passes[i] samples per pixel for jobs[i]; kernel 1 = plain, 2 = wavefront.
+// passes[i] samples per pixel for jobs[i]; kernel 1 = plain, 2 = wavefront,
+// 0 = the wavefront, or for few samples a thread per sample.
 int render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32_t* passes, int kernel,
                 int tile_pixels, int blocks_per_sm, bool count);
 // Wavefront form; `slots` path slots per launch (0 = context default).
+// by_size: launches of few samples take a thread per sample instead.
 int render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32_t* passes, int slots,
-                     int blocks_per_sm, bool count);
+                     int blocks_per_sm, bool count, bool by_size);
 }  // namespace vt

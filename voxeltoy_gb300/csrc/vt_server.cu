@@ -258,7 +258,7 @@ void vt_server::run() {
     }
     vt::Range round_range("vt.server_round");
     const double t0 = now_s();
-    int rc = render_jobs(&lane, jobs.data(), (int32_t)jobs.size(), passes.data(), 2, opts.path_slots, 0, false);
+    int rc = render_jobs(&lane, jobs.data(), (int32_t)jobs.size(), passes.data(), 0, opts.path_slots, 0, false);
     if (rc == VT_OK && cudaStreamSynchronize(lane.stream) != cudaSuccess) rc = VT_EDEVICE;
     const double t1 = now_s();
     std::unique_lock<std::mutex> g(mu);
@@ -305,7 +305,6 @@ extern "C" int vt_server_create(vt_context* ctx, const vt_server_opts* opts, vt_
   vt_context& L = s->lane;
   L.device = ctx->device;
   L.sm_count = ctx->sm_count;
-  L.kernel = 2;
   L.log_fn = ctx->log_fn;
   L.log_user = ctx->log_user;
   // the rounds take the creating context's launch shape (lanes, DDA kernel

@@ -450,11 +450,20 @@ done:
 
 VT_D bool bricks_444(const Grid& g) { return g.shx == 2 && g.shy == 2 && g.shz == 2; }
 
-// The DDA loop for the grid's brick shape (the 4x4x4 loop when it applies).
-template <bool kCount, bool kVote = false>
-VT_D void dda_advance(const Grid& g, Dda& s, int budget, Cnt<kCount>& cnt, int vote_min = 0) {
-  if (bricks_444(g)) dda_steps<kCount, kVote, true>(g, s, budget, cnt, vote_min);
-  else dda_steps<kCount, kVote, false>(g, s, budget, cnt, vote_min);
+// One whole segment that dda_begin set up, in the per-lane kernels: the
+// counted loop, or without event counts the 4x4x4 loop where the grid's bricks
+// have that shape.
+template <bool kCount>
+VT_D void dda_finish(const Grid& g, Dda& s, Cnt<kCount>& cnt) {
+  if (s.state != DDA_RUNNING) return;
+  if (!bricks_444(g)) {
+    dda_steps<kCount, false, false>(g, s, 0x7fffffff, cnt, 0);
+  } else if constexpr (kCount) {
+    dda_steps<kCount, false, true>(g, s, 0x7fffffff, cnt, 0);
+  } else {
+    dda_end_stuck(g, s);
+    if (s.state == DDA_RUNNING) dda_steps_444<false>(g, s, 1 << 30, 0);
+  }
 }
 
 // traverse (dda.h:63-79): voxel hit, or with the ground quirk an exit below y = 0.
@@ -1052,7 +1061,7 @@ VT_D float4 edit_sample(const Frame& F, const JobDev& J, int px, int py, int sam
   float t_enter;
   if (!path_start(F, J, p, px, py, sample, cnt, t_enter)) return make_float4(p.L.x, p.L.y, p.L.z, 1.0f);
   dda_begin(g, s, p.ro + t_enter * p.rd, p.rd);
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  dda_finish(g, s, cnt);
   const bool hit = dda_hit(F, s);
   Basis b;
   if (hit) b = voxel_basis(F, s.x, s.y, s.z, p.ro, p.rd, !(F.quirks & Q_UNGUARDED));
@@ -1080,7 +1089,7 @@ VT_D float4 edit_sample(const Frame& F, const JobDev& J, int px, int py, int sam
   lighting = sqrtf(lighting);
   cnt.add(C_SEGMENTS, 1);
   dda_begin(g, s, b.position, mk3(-1.0f, 1.0f, 1.0f));            // :133: -lightDirection
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  dda_finish(g, s, cnt);
   if (dda_hit(F, s)) lighting = lighting * 0.5f;
   const v3 radiance = albedo * lighting;
   return make_float4(radiance.x, radiance.y, radiance.z, 1.0f);
@@ -1097,7 +1106,7 @@ VT_D float4 trace_sample(const Frame& F, const JobDev& J, int px, int py, int sa
   float t_enter;
   if (!path_start(F, J, p, px, py, sample, cnt, t_enter)) return path_output(F, p);
   dda_begin(g, s, p.ro + t_enter * p.rd, p.rd);
-  if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+  dda_finish(g, s, cnt);
   if (first_hit) {
     const bool h = dda_hit(F, s);
     first_hit->x = s.x; first_hit->y = s.y; first_hit->z = s.z;
@@ -1110,11 +1119,11 @@ VT_D float4 trace_sample(const Frame& F, const JobDev& J, int px, int py, int sa
   }
   while (ext_end(F, J, p, seg_end(s), cnt)) {
     dda_begin(g, s, p.ro, p.sd);
-    if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+    dda_finish(g, s, cnt);
     shadow_end(F, p, seg_end(s));
     if (!p.has_cont) break;
     dda_begin(g, s, p.ro, p.rd);
-    if (s.state == DDA_RUNNING) dda_advance(g, s, 0x7fffffff, cnt);
+    dda_finish(g, s, cnt);
   }
   return path_output(F, p);
 }
