@@ -294,29 +294,31 @@ static void scene_bounds(vt_scene* s) {
   }
 }
 
-// Emissive-list pruning with the reference's swap-with-last removal order
-// (Renderer::pruneInteriorEmissiveVoxels, src/renderer/import.cpp:180-203);
-// the neighbour tests run on the GPU.
-// `on_device` (nullable): the same list already in device memory.
-static int prune_emissive(vt_context* ctx, vt_scene* s, std::vector<int32_t>& list,
-                          const int32_t* on_device = nullptr) {
+static EmissiveVolume emissive_volume(const vt_scene* s, bool prune) {
+  EmissiveVolume V;
+  V.rx = s->res[0]; V.ry = s->res[1]; V.rz = s->res[2];
+  V.prune = prune ? 1 : 0;
+  V.n = (int64_t)V.rx * V.ry * V.rz;
+  V.m_x = udiv_magic((uint32_t)V.rx);
+  V.m_xy = udiv_magic((uint32_t)V.rx * (uint32_t)V.ry);
+  return V;
+}
+
+// Pruning of a caller's emissive list with the reference's swap-with-last
+// removal order (Renderer::pruneInteriorEmissiveVoxels,
+// src/renderer/import.cpp:180-203); the neighbour tests run on the GPU.
+static int prune_emissive(vt_context* ctx, vt_scene* s, std::vector<int32_t>& list) {
   if (list.empty()) return VT_OK;
   const int64_t n = (int64_t)list.size();
   int32_t* d_list = nullptr;
   uint8_t* d_keep = nullptr;
-  int rc = VT_OK;
-  if (!on_device) {
-    rc = ctx->alloc((void**)&d_list, sizeof(int32_t) * n);
-    if (rc != VT_OK) return rc;
-  }
+  int rc = ctx->alloc((void**)&d_list, sizeof(int32_t) * n);
+  if (rc != VT_OK) return rc;
   rc = ctx->alloc((void**)&d_keep, (size_t)n);
   if (rc != VT_OK) { ctx->release(d_list); return rc; }
   std::vector<uint8_t> keep(n);
-  cudaError_t e = cudaSuccess;
-  if (!on_device)
-    e = cudaMemcpyAsync(d_list, list.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx->stream);
-  const int32_t* dl = on_device ? on_device : d_list;
-  if (e == cudaSuccess) e = launch_emissive_flags(s->grid, s->res[0], s->res[1], s->res[2], dl, n, d_keep, ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(d_list, list.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = launch_emissive_flags(s->grid, emissive_volume(s, true), d_list, n, d_keep, ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(keep.data(), d_keep, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   ctx->release(d_list);
@@ -341,6 +343,41 @@ static int prune_emissive(vt_context* ctx, vt_scene* s, std::vector<int32_t>& li
   return VT_OK;
 }
 
+// The emissive list of the voxels with em[entry] != 0, found and pruned on
+// the device, in place of the scene's previous list.
+static int discover_emissive(vt_context* ctx, vt_scene* s, const uint8_t (&em)[256], bool prune) {
+  const EmissiveVolume V = emissive_volume(s, prune);
+  const int64_t chunks = emissive_chunks(V.n);
+  void* tmp = nullptr;
+  int rc = ctx->alloc(&tmp, 256 + sizeof(unsigned long long) * (size_t)(chunks + 1));
+  if (rc != VT_OK) return rc;
+  uint8_t* d_em = (uint8_t*)tmp;
+  unsigned long long* d_counts = (unsigned long long*)((char*)tmp + 256);
+  unsigned long long totals = 0;   // pageable: the read has completed when the copy returns
+  cudaError_t e = cudaMemcpyAsync(d_em, em, 256, cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = launch_emissive_count(s->grid, V, d_em, d_counts, ctx->stream);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&totals, d_counts + chunks, sizeof(totals), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e != cudaSuccess) { ctx->release(tmp); return cuda_fail(e, "emissive discovery"); }
+  const int64_t found = (int64_t)(totals & 0xffffffffull), listed = (int64_t)(totals >> 32);
+  const int64_t n_movers = std::min(listed, found - listed);
+  int32_t *d_out = nullptr, *d_movers = nullptr;
+  rc = ctx->alloc((void**)&d_out, sizeof(int32_t) * (size_t)std::max<int64_t>(listed, 1));
+  if (rc == VT_OK && n_movers > 0) rc = ctx->alloc((void**)&d_movers, sizeof(int32_t) * (size_t)n_movers);
+  if (rc == VT_OK) {
+    e = launch_emissive_write(s->grid, V, d_em, d_counts, d_out, listed, d_movers, ctx->stream);
+    if (e != cudaSuccess) rc = cuda_fail(e, "emissive discovery");
+  }
+  ctx->release(d_movers);
+  ctx->release(tmp);
+  if (rc != VT_OK) { ctx->release(d_out); return rc; }
+  if (prune && found > 0) ctx->log("Pruned emissive voxels: %lld/%lld", (long long)(found - listed), (long long)found);
+  ctx->release(s->emissive);
+  s->emissive = d_out;
+  s->n_emissive = listed;
+  return VT_OK;
+}
+
 // The scene's emissive list: discovered from the palette
 // (VT_SCENE_AUTO_EMISSIVE, in voxel order) or the caller's indices, pruned
 // when VT_SCENE_PRUNE_EMISSIVE asks, uploaded in place of the previous list.
@@ -362,36 +399,7 @@ static int scene_emissive(vt_context* ctx, vt_scene* s, const int32_t* emissive,
     }
     bool lit = false;   // no emitting entry: an empty list without a pass over the grid
     for (int i = 1; i <= n_palette; ++i) lit = lit || em[i] != 0;
-    // voxel order, found on the device (two passes over the grid)
-    const int64_t chunks = lit ? emissive_chunks(nvox) : 0;
-    void* tmp = nullptr;
-    rc = ctx->alloc(&tmp, 256 + sizeof(uint32_t) * (size_t)(chunks + 1));
-    if (rc != VT_OK) return rc;
-    uint8_t* d_em = (uint8_t*)tmp;
-    uint32_t* d_counts = (uint32_t*)((char*)tmp + 256);
-    uint32_t total = 0;   // pageable: the read has completed when the copy returns
-    cudaError_t e = cudaSuccess;
-    if (lit) {
-      e = cudaMemcpyAsync(d_em, em, 256, cudaMemcpyHostToDevice, ctx->stream);
-      if (e == cudaSuccess) e = launch_emissive_count(s->grid, nvox, d_em, d_counts, ctx->stream);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&total, d_counts + chunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream);
-    }
-    int32_t* d_out = nullptr;
-    if (e == cudaSuccess && total > 0) {
-      rc = ctx->alloc((void**)&d_out, sizeof(int32_t) * (size_t)total);
-      if (rc != VT_OK) { ctx->release(tmp); return rc; }
-      list.resize(total);
-      e = launch_emissive_write(s->grid, nvox, d_em, d_counts, d_out, ctx->stream);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(list.data(), d_out, sizeof(int32_t) * (size_t)total, cudaMemcpyDeviceToHost, ctx->stream);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    }
-    if (e == cudaSuccess && (flags & VT_SCENE_PRUNE_EMISSIVE)) rc = prune_emissive(ctx, s, list, d_out);
-    ctx->release(d_out);
-    ctx->release(tmp);
-    if (e != cudaSuccess) return cuda_fail(e, "emissive discovery");
-    if (rc != VT_OK) return rc;
+    if (lit) return discover_emissive(ctx, s, em, (flags & VT_SCENE_PRUNE_EMISSIVE) != 0);
   } else if (n_emissive > 0) {
     VT_CHECK_ARG(emissive, "emissive_indices is null");
     list.assign(emissive, emissive + n_emissive);
@@ -733,20 +741,19 @@ vt_env::~vt_env() {
   ctx->release(cdf_v);
 }
 
-// Scratch layout of an environment build: nine offsets into one buffer.
-static size_t env_scratch_bytes(int32_t w, int32_t h, size_t (&offs)[9]) {
+// Scratch layout of an environment build: eight offsets into one buffer.
+static size_t env_scratch_bytes(int32_t w, int32_t h, size_t (&offs)[8]) {
   const size_t n = (size_t)w * h;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o += (bytes + 255) & ~(size_t)255; return at; };
   offs[0] = take(sizeof(float) * n);                 // lum
-  offs[1] = take(sizeof(float) * n);                 // tmp
-  offs[2] = take(sizeof(float) * n);                 // func
-  offs[3] = take(sizeof(float) * h);                 // sin
-  offs[4] = take(sizeof(double) * (size_t)h * (w + 1));  // row prefixes
-  offs[5] = take(sizeof(double) * h);                // row integrals
-  offs[6] = take(sizeof(double) * (h + 1));          // marginal prefixes
-  offs[7] = take(sizeof(float) * 3 * n);             // rgb input
-  offs[8] = take(2 * sizeof(uint32_t));              // integral, first non-finite texel
+  offs[1] = take(sizeof(float) * n);                 // func
+  offs[2] = take(sizeof(float) * h);                 // sin
+  offs[3] = take(sizeof(double) * (size_t)h * (w + 1));  // row prefixes
+  offs[4] = take(sizeof(double) * h);                // row integrals
+  offs[5] = take(sizeof(double) * (h + 1));          // marginal prefixes
+  offs[6] = take(sizeof(float) * 3 * n);             // rgb input
+  offs[7] = take(2 * sizeof(uint32_t));              // integral, first non-finite texel
   return o;
 }
 
@@ -754,12 +761,11 @@ static EnvScratch env_scratch(void* base, const size_t* offs) {
   char* b = (char*)base;
   EnvScratch S;
   S.lum = (float*)(b + offs[0]);
-  S.tmp = (float*)(b + offs[1]);
-  S.func = (float*)(b + offs[2]);
-  S.sin_theta = (float*)(b + offs[3]);
-  S.row_pre = (double*)(b + offs[4]);
-  S.row_int = (double*)(b + offs[5]);
-  S.marg_pre = (double*)(b + offs[6]);
+  S.func = (float*)(b + offs[1]);
+  S.sin_theta = (float*)(b + offs[2]);
+  S.row_pre = (double*)(b + offs[3]);
+  S.row_int = (double*)(b + offs[4]);
+  S.marg_pre = (double*)(b + offs[5]);
   return S;
 }
 
@@ -796,7 +802,7 @@ extern "C" int vt_env_create_image_ex(vt_context* ctx, const float* rgb, int32_t
   int rc = ctx->alloc((void**)&env->texels, sizeof(uint2) * n);
   if (rc == VT_OK) rc = ctx->alloc((void**)&env->cdf_u, sizeof(float) * (size_t)(cw + 1) * ch);
   if (rc == VT_OK) rc = ctx->alloc((void**)&env->cdf_v, sizeof(float) * (size_t)(ch + 1));
-  size_t offs[9];
+  size_t offs[8];
   const size_t sb = env_scratch_bytes(w, h, offs);
   if (rc == VT_OK) rc = ctx->ensure_scratch(sb);   // kept by the context for the next build
   if (rc != VT_OK) { delete env; return rc; }
@@ -805,8 +811,8 @@ extern "C" int vt_env_create_image_ex(vt_context* ctx, const float* rgb, int32_t
   // row weights sin(pi (y + 0.5) / h) of the CDF image, as calculateImageIntegral computes them (image.cpp:366)
   std::vector<float> sin_theta(ch);
   for (int y = 0; y < ch; ++y) sin_theta[y] = (float)std::sin(M_PI * (double)((float)y + 0.5f) / (double)(float)ch);
-  float* d_rgb = (float*)((char*)scratch + offs[7]);
-  uint32_t* d_out = (uint32_t*)((char*)scratch + offs[8]);   // integral bits, first non-finite texel
+  float* d_rgb = (float*)((char*)scratch + offs[6]);
+  uint32_t* d_out = (uint32_t*)((char*)scratch + offs[7]);   // integral bits, first non-finite texel
   uint32_t res[2] = {0u, 0u};   // pageable: the read has completed when the copy returns
   cudaError_t e = cudaMemcpyAsync(d_rgb, rgb, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess)
@@ -2177,7 +2183,7 @@ extern "C" int vt_diag_cdf_from_function(vt_context* ctx, const float* func, int
                                          float* cdf_v, float* integral) {
   VT_CHECK_ARG(ctx && func && cdf_u && cdf_v && w > 0 && h > 0, "bad argument");
   cudaSetDevice(ctx->device);
-  size_t offs[9];
+  size_t offs[8];
   const size_t sb = env_scratch_bytes(w, h, offs);
   const size_t extra = ((sizeof(float) * (size_t)(w + 1) * h + 255) & ~(size_t)255) +
                        ((sizeof(float) * (size_t)(h + 2) + 255) & ~(size_t)255) + 256;

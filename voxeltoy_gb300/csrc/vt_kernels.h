@@ -164,23 +164,30 @@ cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t 
 cudaError_t launch_build_bricks(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
                                 unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, const BrickShape& sh,
                                 unsigned long long* max_entry, cudaStream_t st);
-cudaError_t launch_emissive_flags(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
-                                  const int32_t* emissive, int64_t n, uint8_t* keep, cudaStream_t st);
-// Emissive voxels in increasing index order, in two launches:
-// launch_emissive_count leaves in counts[0..chunks) each chunk's first output
-// position and in counts[chunks] the total (counts holds chunks + 1 words,
-// chunks = emissive_chunks(n_voxels)); launch_emissive_write then writes the
-// total indices into out.
+// A volume as the emissive passes see it.
+struct EmissiveVolume {
+  int32_t rx, ry, rz;
+  int32_t prune;             // list only voxels with a visible face
+  int64_t n;                 // rx * ry * rz
+  uint64_t m_x, m_xy;        // udiv_magic of rx and rx * ry
+};
+cudaError_t launch_emissive_flags(const uint8_t* grid, const EmissiveVolume& V, const int32_t* emissive, int64_t n,
+                                  uint8_t* keep, cudaStream_t st);
+// A volume's emissive list, in two launches: launch_emissive_count leaves in
+// counts (chunks + 1 words, chunks = emissive_chunks(V.n)) each chunk's
+// offsets and in counts[chunks] the emissive voxels (low 32 bits) and the
+// listed ones (high); launch_emissive_write then writes the listed ones into
+// out.  movers: scratch of min(listed, emissive - listed) ints, null if that is 0.
 int64_t emissive_chunks(int64_t n_voxels);
-cudaError_t launch_emissive_count(const uint8_t* grid, int64_t n_voxels, const uint8_t* emissive_entry,
-                                  uint32_t* counts, cudaStream_t st);
-cudaError_t launch_emissive_write(const uint8_t* grid, int64_t n_voxels, const uint8_t* emissive_entry,
-                                  const uint32_t* offsets, int32_t* out, cudaStream_t st);
+cudaError_t launch_emissive_count(const uint8_t* grid, const EmissiveVolume& V, const uint8_t* emissive_entry,
+                                  unsigned long long* counts, cudaStream_t st);
+cudaError_t launch_emissive_write(const uint8_t* grid, const EmissiveVolume& V, const uint8_t* emissive_entry,
+                                  const unsigned long long* counts, int32_t* out, int64_t listed, int32_t* movers,
+                                  cudaStream_t st);
 // Scratch buffers of the environment build (device memory, caller-owned).
 struct EnvScratch {
   float* lum;        // w*h luminance of the FP16 texels
-  float* tmp;        // w*h horizontal blur
-  float* func;       // w*h sampled function: blurred luminance * sin(theta)
+  float* func;       // w*h sampled function (launch_cdf's input)
   float* sin_theta;  // h row weights sin(pi (y + 0.5) / h), computed on the host
   double* row_pre;   // h*(w+1) row prefix sums
   double* row_int;   // h row integrals

@@ -11,55 +11,63 @@ namespace vt {
 
 // ------------------------------------------------------------- bit-bricks
 // One thread per brick of the padded brick grid (one border brick on every
-// side).  Voxels outside the volume read as occupied, so the DDA stops on
-// the first voxel beyond the volume without a separate bounds test.
+// side), a warp along x, blocks of eight rows, grid y over brick slices.
+// Voxels outside the volume read as occupied, so the DDA stops on the first
+// voxel beyond the volume without a separate bounds test.
 //
 // With `max_entry`, the largest palette entry of the volume is atomically
 // max-ed into *max_entry (the host checks it against the palette size).
-__global__ void k_build_bricks(const uint8_t* __restrict__ grid, int32_t rx, int32_t ry, int32_t rz,
-                               unsigned long long* __restrict__ bricks, int32_t bx, int32_t by, int32_t bz,
-                               const BrickShape sh, unsigned long long* max_entry) {
-  const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t px = bx + 2, py = by + 2, pz = bz + 2;
+// Bound by the read of the volume; border bricks are written without a look
+// at their voxels and indices take no division (a thread per brick of the
+// flattened array, with both, took 30 us for 256^3, now 21).
+constexpr int kBrickRows = 8;
+__global__ void __launch_bounds__(32 * kBrickRows) k_build_bricks(const uint8_t* __restrict__ grid, int32_t rx,
+                                                                  int32_t ry, int32_t rz,
+                                                                  unsigned long long* __restrict__ bricks, int32_t bx,
+                                                                  int32_t by, int32_t bz, const BrickShape sh,
+                                                                  unsigned long long* max_entry) {
+  const int px = bx + 2, py = by + 2;
+  const int iy = blockIdx.x * kBrickRows + threadIdx.y;
   unsigned top = 0;
-  if (b < px * py * pz) {
-    const int ex = 1 << sh.sx, ey = 1 << sh.sy, ez = 1 << sh.sz;
-    const int x0 = ((int)(b % px) - 1) * ex;
-    const int y0 = ((int)((b / px) % py) - 1) * ey;
-    const int z0 = ((int)(b / (px * py)) - 1) * ez;
-    unsigned long long w = 0ull;
-    unsigned tops = 0u;   // byte-wise maximum of the word rows
-    // 4x4x4 bricks: rows of four voxels as one aligned 32-bit word where the
-    // brick's x range lies inside the volume and rows start on 4-byte
-    // boundaries; the sixteen row loads are independent
-    const bool words = sh.sx == 2 && sh.sy == 2 && (rx & 3) == 0 && x0 >= 0 && x0 + 4 <= rx;
-    if (words) {
+  for (int iz = blockIdx.y; iz < bz + 2; iz += gridDim.y)
+    for (int ix = threadIdx.x; ix < px && iy < py; ix += 32) {
+      unsigned long long w = 0ull;
+      const int ex = 1 << sh.sx, ey = 1 << sh.sy, ez = 1 << sh.sz;
+      const int x0 = (ix - 1) * ex, y0 = (iy - 1) * ey, z0 = (iz - 1) * ez;
+      if (ix == 0 || iy == 0 || iz == 0 || ix > bx || iy > by || iz > bz) {
+        w = ~0ull;   // border
+      } else if (sh.sx == 2 && sh.sy == 2 && (rx & 3) == 0) {
+        // 4x4x4 bricks: rows of four voxels as one aligned 32-bit word where
+        // rows start on 4-byte boundaries; the sixteen loads are independent
+        unsigned tops = 0u;   // byte-wise maximum of the word rows
 #pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        const int y = y0 + (r & 3), z = z0 + (r >> 2);
-        const bool in = y >= 0 && z >= 0 && y < ry && z < rz;
-        const uint32_t v4 =
-            in ? *reinterpret_cast<const uint32_t*>(grid + (size_t)x0 + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z))
-               : 0u;
-        tops = __vmaxu4(tops, v4);
-        uint32_t m = __vcmpne4(v4, 0u) & 0x01010101u;   // bit 0 of each non-zero byte
-        m = (m | (m >> 7) | (m >> 14) | (m >> 21)) & 0xfu;
-        w |= (unsigned long long)(in ? m : 0xfu) << (4 * r);   // rows outside the volume read as set
+        for (int r = 0; r < 16; ++r) {
+          const int y = y0 + (r & 3), z = z0 + (r >> 2);
+          const bool in = y < ry && z < rz;
+          const uint32_t v4 =
+              in ? *reinterpret_cast<const uint32_t*>(grid + (size_t)x0 + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z))
+                 : 0u;
+          tops = __vmaxu4(tops, v4);
+          uint32_t m = __vcmpne4(v4, 0u) & 0x01010101u;   // bit 0 of each non-zero byte
+          m = (m | (m >> 7) | (m >> 14) | (m >> 21)) & 0xfu;
+          w |= (unsigned long long)(in ? m : 0xfu) << (4 * r);   // rows outside the volume read as set
+        }
+        for (int k = 0; k < 32; k += 8) top = max(top, (tops >> k) & 0xffu);
+      } else {
+        for (int k = 0; k < 64; ++k) {
+          const int x = x0 + (k & (ex - 1)), y = y0 + ((k >> sh.sx) & (ey - 1)), z = z0 + (k >> (sh.sx + sh.sy));
+          const bool outside = x >= rx || y >= ry || z >= rz;
+          const unsigned v = outside ? 0u : grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)];
+          top = v > top ? v : top;
+          if (outside || v != 0) w |= 1ull << k;
+        }
       }
-    } else {
-      for (int k = 0; k < 64; ++k) {
-        const int x = x0 + (k & (ex - 1)), y = y0 + ((k >> sh.sx) & (ey - 1)), z = z0 + (k >> (sh.sx + sh.sy));
-        const bool outside = x < 0 || y < 0 || z < 0 || x >= rx || y >= ry || z >= rz;
-        const unsigned v = outside ? 0u : grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)];
-        top = v > top ? v : top;
-        if (outside || v != 0) w |= 1ull << k;
-      }
+      bricks[(int64_t)ix + (int64_t)px * ((int64_t)iy + (int64_t)py * iz)] = w;
     }
-    for (int k = 0; k < 32; k += 8) top = max(top, (tops >> k) & 0xffu);
-    bricks[b] = w;
-  }
+  // an atomic only where it would raise the maximum
   top = __reduce_max_sync(0xffffffffu, top);
-  if (max_entry && (threadIdx.x & 31) == 0 && top) atomicMax(max_entry, (unsigned long long)top);
+  if (max_entry && threadIdx.x == 0 && top > *(volatile unsigned long long*)max_entry)
+    atomicMax(max_entry, (unsigned long long)top);
 }
 
 // One voxel edit: its grid entry and its bit in the padded brick grid.
@@ -82,65 +90,75 @@ cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t 
 cudaError_t launch_build_bricks(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
                                 unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, const BrickShape& sh,
                                 unsigned long long* max_entry, cudaStream_t st) {
-  const int64_t nb = (int64_t)(bx + 2) * (by + 2) * (bz + 2);
-  k_build_bricks<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(grid, rx, ry, rz, bricks, bx, by, bz, sh, max_entry);
+  const dim3 blocks((unsigned)((by + 2 + kBrickRows - 1) / kBrickRows), (unsigned)std::min(bz + 2, 65535));
+  k_build_bricks<<<blocks, dim3(32, kBrickRows), 0, st>>>(grid, rx, ry, rz, bricks, bx, by, bz, sh, max_entry);
   return cudaGetLastError();
 }
 
 // --------------------------------------------------------- emissive voxels
-// keep[i] = 1 if emissive voxel i has an empty or out-of-range 6-neighbour
-// (anyVisibleFace, src/renderer/import.cpp:133-178).
-__global__ void k_emissive_flags(const uint8_t* __restrict__ grid, int32_t rx, int32_t ry, int32_t rz,
-                                 const int32_t* __restrict__ emissive, int64_t n, uint8_t* __restrict__ keep) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t v = emissive[i];
-  const int64_t sxy = (int64_t)rx * ry;
-  const int z = (int)(v / sxy);
-  const int64_t r = v - (int64_t)z * sxy;
-  const int y = (int)(r / rx);
-  const int x = (int)(r - (int64_t)y * rx);
-  const int off[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-  bool visible = false;
-  for (int k = 0; k < 6 && !visible; ++k) {
-    const int nx = x + off[k][0], ny = y + off[k][1], nz = z + off[k][2];
-    if (nx < 0 || nx >= rx || ny < 0 || ny >= ry || nz < 0 || nz >= rz) { visible = true; break; }
-    if (grid[(size_t)nx + (size_t)rx * ((size_t)ny + (size_t)ry * (size_t)nz)] == 0) visible = true;
-  }
-  keep[i] = visible ? 1 : 0;
+// Whether voxel v has an empty or out-of-range 6-neighbour (anyVisibleFace,
+// src/renderer/import.cpp:133-178).
+__device__ __forceinline__ bool visible_face(const uint8_t* __restrict__ grid, const EmissiveVolume& V, int64_t v) {
+  const uint32_t i = (uint32_t)v;   // fewer than 2^31 voxels
+  const uint32_t z = udiv(i, V.m_xy), r = i - z * (uint32_t)(V.rx * V.ry);
+  const uint32_t y = udiv(r, V.m_x), x = r - y * (uint32_t)V.rx;
+  if (x == 0 || y == 0 || z == 0 || x == (uint32_t)V.rx - 1u || y == (uint32_t)V.ry - 1u || z == (uint32_t)V.rz - 1u)
+    return true;
+  const size_t sy = (size_t)V.rx, sz = (size_t)V.rx * V.ry;
+  const uint8_t* g = grid + v;
+  return g[1] == 0 || *(g - 1) == 0 || g[sy] == 0 || *(g - sy) == 0 || g[sz] == 0 || *(g - sz) == 0;
 }
 
-cudaError_t launch_emissive_flags(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
-                                  const int32_t* emissive, int64_t n, uint8_t* keep, cudaStream_t st) {
+// keep[i] = 1 if listed emissive voxel i has a visible face.
+__global__ void k_emissive_flags(const uint8_t* __restrict__ grid, const EmissiveVolume V,
+                                 const int32_t* __restrict__ emissive, int64_t n, uint8_t* __restrict__ keep) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) keep[i] = visible_face(grid, V, emissive[i]) ? 1 : 0;
+}
+
+cudaError_t launch_emissive_flags(const uint8_t* grid, const EmissiveVolume& V, const int32_t* emissive, int64_t n,
+                                  uint8_t* keep, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  k_emissive_flags<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(grid, rx, ry, rz, emissive, n, keep);
+  k_emissive_flags<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(grid, V, emissive, n, keep);
   return cudaGetLastError();
 }
 
-// Linear indices of voxels whose palette entry emits (emissive_entry[g] != 0),
-// in increasing order: the volume is cut into chunks of kEmChunk voxels; one
-// kernel counts each chunk's emissive voxels, one block turns the counts into
-// chunk offsets, and a second pass over the chunks writes each chunk's
-// indices from its offset, rows of 256 voxels at a time in voxel order.
+// Emissive list of a volume (the voxels whose palette entry emits,
+// emissive_entry[g] != 0), pruned on request to those with a visible face, in
+// the order that the reference's sequential removal leaves: the full list is
+// in voxel order, and each removed element is replaced by the last one still
+// in it (import.cpp:180-203).  With K elements kept, that is: a kept element
+// whose place in the full list is below K stays there, and the kept ones from
+// K on, last first, fill the removed places below K in increasing order.
+//
+// The volume is cut into chunks of kEmChunk voxels.  k_emissive_count counts
+// each chunk's emissive and kept voxels, one block turns the counts into
+// offsets, and k_emissive_write visits the chunks again and writes every kept
+// element below K to its place, ~r to the r-th removed place below K, and the
+// kept ones from K on to the mover list by their rank from the end;
+// k_emissive_fill puts mover r in the place that holds ~r.  16
+// voxels per thread and load, one block-wide prefix a chunk: reading the
+// volume a byte per thread in rows with a prefix each took 56 us of a 256^3
+// volume (now 18), and the pruning on the host, with its copies both ways, 0.4
+// ms of its 0.64 ms load (now 0.22).
 constexpr int kEmThreads = 256;
-constexpr int kEmRows = 16;
-constexpr int64_t kEmChunk = (int64_t)kEmThreads * kEmRows;
+constexpr int64_t kEmChunk = (int64_t)kEmThreads * 16;
 
 // Exclusive prefix of `v` over the block (kThreads threads); *total gets the sum.
-template <int kThreads = kEmThreads>
-__device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
+template <class V, int kThreads = kEmThreads>
+__device__ __forceinline__ V block_prefix(V v, V* warp_sums, V* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+  V x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    const V y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
   }
   if (lane == 31) warp_sums[warp] = x;
   __syncthreads();
-  uint32_t before = 0, all = 0;
+  V before = 0, all = 0;
   for (int w = 0; w < kThreads / 32; ++w) {
-    before += w < warp ? warp_sums[w] : 0u;
+    before += w < warp ? warp_sums[w] : (V)0;
     all += warp_sums[w];
   }
   __syncthreads();   // warp_sums is reused by the next call
@@ -148,77 +166,122 @@ __device__ __forceinline__ uint32_t block_prefix(uint32_t v, uint32_t* warp_sums
   return before + x - v;
 }
 
-__global__ void k_emissive_count(const uint8_t* __restrict__ grid, int64_t n_voxels,
-                                 const uint8_t* __restrict__ emissive_entry, uint32_t* __restrict__ counts) {
-  __shared__ uint8_t s_em[256];
-  __shared__ uint32_t s_warp[kEmThreads / 32];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) s_em[i] = emissive_entry[i];
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kEmChunk;
-  uint32_t c = 0;
-  for (int r = 0; r < kEmRows; ++r) {
-    const int64_t i = base + (int64_t)r * kEmThreads + threadIdx.x;
-    if (i < n_voxels && s_em[grid[i]]) ++c;
+// The 16 voxels of this thread in its chunk: bit i of *em set if voxel
+// base + i emits, of *keep if it is also listed after pruning.
+__device__ __forceinline__ void emissive_bits(const uint8_t* __restrict__ grid, const EmissiveVolume& V, int64_t base,
+                                              const uint8_t* s_em, uint32_t* em, uint32_t* keep) {
+  uint32_t e = 0u, k = 0u;
+  if (base + 16 <= V.n) {   // base is a multiple of 16, the grid starts on a 16-byte boundary
+    const uint4 q = *(const uint4*)(grid + base);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    if (q.x | q.y | q.z | q.w) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) e |= (uint32_t)s_em[(w[i >> 2] >> (8 * (i & 3))) & 0xffu] << i;
+    }
+  } else {
+    for (int i = 0; i < 16 && base + i < V.n; ++i) e |= (uint32_t)s_em[grid[base + i]] << i;
   }
-  uint32_t total;
-  block_prefix(c, s_warp, &total);
-  if (threadIdx.x == 0) counts[blockIdx.x] = total;
+  for (uint32_t left = e; left; left &= left - 1u) {
+    const int i = __ffs(left) - 1;
+    if (!V.prune || visible_face(grid, V, base + i)) k |= 1u << i;
+  }
+  *em = e;
+  *keep = k;
 }
 
-// In place: counts[0..n) -> exclusive offsets, counts[n] = total.  One block
-// of kScanThreads threads, each over a contiguous run of counts.
+__device__ __forceinline__ void emissive_table(const uint8_t* emissive_entry, uint8_t* s_em) {
+  for (int i = threadIdx.x; i < 256; i += blockDim.x) s_em[i] = emissive_entry[i] ? 1 : 0;
+  __syncthreads();
+}
+
+// counts[chunk]: emissive voxels in the low, kept ones in the high 32 bits.
+__global__ void __launch_bounds__(kEmThreads) k_emissive_count(const uint8_t* __restrict__ grid, const EmissiveVolume V,
+                                                               const uint8_t* __restrict__ emissive_entry,
+                                                               unsigned long long* __restrict__ counts) {
+  __shared__ uint8_t s_em[256];
+  __shared__ uint32_t s_warp[kEmThreads / 32];
+  emissive_table(emissive_entry, s_em);
+  uint32_t em, keep;
+  emissive_bits(grid, V, (int64_t)blockIdx.x * kEmChunk + 16 * threadIdx.x, s_em, &em, &keep);
+  uint32_t total;   // a chunk holds at most 4096 of either
+  block_prefix((uint32_t)__popc(em) | ((uint32_t)__popc(keep) << 16), s_warp, &total);
+  if (threadIdx.x == 0) counts[blockIdx.x] = (unsigned long long)(total & 0xffffu) | ((unsigned long long)(total >> 16) << 32);
+}
+
+// In place: counts[0..n) -> exclusive offsets of both counts, counts[n] = the
+// totals.  One block of kScanThreads threads, each over a contiguous run.
 constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) k_emissive_offsets(uint32_t* counts, int64_t n) {
-  __shared__ uint32_t s_warp[kScanThreads / 32];
+__global__ void __launch_bounds__(kScanThreads) k_emissive_offsets(unsigned long long* counts, int64_t n) {
+  __shared__ unsigned long long s_warp[kScanThreads / 32];
   const int64_t per = (n + kScanThreads - 1) / kScanThreads;
   const int64_t b = (int64_t)threadIdx.x * per, e = b + per < n ? b + per : n;
-  uint32_t sum = 0;
-  for (int64_t i = b; i < e; ++i) sum += counts[i];
-  uint32_t total;
-  uint32_t run = block_prefix<kScanThreads>(sum, s_warp, &total);
+  unsigned long long sum = 0;
+  for (int64_t i = b; i < e; ++i) sum += counts[i];   // either half stays below 2^31
+  unsigned long long total;
+  unsigned long long run = block_prefix<unsigned long long, kScanThreads>(sum, s_warp, &total);
   for (int64_t i = b; i < e; ++i) {
-    const uint32_t c = counts[i];
+    const unsigned long long c = counts[i];
     counts[i] = run;
     run += c;
   }
   if (threadIdx.x == 0) counts[n] = total;
 }
 
-__global__ void k_emissive_write(const uint8_t* __restrict__ grid, int64_t n_voxels,
-                                 const uint8_t* __restrict__ emissive_entry, const uint32_t* __restrict__ offsets,
-                                 int32_t* __restrict__ out) {
+__global__ void __launch_bounds__(kEmThreads) k_emissive_write(const uint8_t* __restrict__ grid, const EmissiveVolume V,
+                                                               const uint8_t* __restrict__ emissive_entry,
+                                                               const unsigned long long* __restrict__ counts,
+                                                               int64_t chunks, int32_t* __restrict__ out,
+                                                               int32_t* __restrict__ movers) {
   __shared__ uint8_t s_em[256];
   __shared__ uint32_t s_warp[kEmThreads / 32];
-  for (int i = threadIdx.x; i < 256; i += blockDim.x) s_em[i] = emissive_entry[i];
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kEmChunk;
-  uint32_t at = offsets[blockIdx.x];
-  for (int r = 0; r < kEmRows; ++r) {
-    const int64_t i = base + (int64_t)r * kEmThreads + threadIdx.x;
-    const bool e = i < n_voxels && s_em[grid[i]];
-    uint32_t total;
-    const uint32_t pre = block_prefix(e ? 1u : 0u, s_warp, &total);
-    if (e) out[at + pre] = (int32_t)i;
-    at += total;
+  const unsigned long long first = counts[blockIdx.x], next = counts[blockIdx.x + 1];
+  if ((uint32_t)first == (uint32_t)next) return;   // nothing emits in this chunk
+  emissive_table(emissive_entry, s_em);
+  const int64_t base = (int64_t)blockIdx.x * kEmChunk + 16 * threadIdx.x;
+  uint32_t em, keep;
+  emissive_bits(grid, V, base, s_em, &em, &keep);
+  uint32_t total;
+  const uint32_t pre = block_prefix((uint32_t)__popc(em) | ((uint32_t)__popc(keep) << 16), s_warp, &total);
+  const uint32_t K = (uint32_t)(counts[chunks] >> 32);
+  uint32_t pos = (uint32_t)first + (pre & 0xffffu), kept = (uint32_t)(first >> 32) + (pre >> 16);
+  for (uint32_t left = em; left; left &= left - 1u) {
+    const int i = __ffs(left) - 1;
+    if ((keep >> i) & 1u) {
+      if (pos < K) out[pos] = (int32_t)(base + i);
+      else movers[K - 1u - kept] = (int32_t)(base + i);   // its rank from the end of the kept ones
+      ++kept;
+    } else if (pos < K) {
+      out[pos] = (int32_t)~(pos - kept);
+    }
+    ++pos;
   }
+}
+
+__global__ void k_emissive_fill(const int32_t* __restrict__ movers, int64_t listed, int32_t* __restrict__ out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= listed) return;
+  const int32_t v = out[i];
+  if (v < 0) out[i] = movers[~v];
 }
 
 int64_t emissive_chunks(int64_t n_voxels) { return (n_voxels + kEmChunk - 1) / kEmChunk; }
 
-cudaError_t launch_emissive_count(const uint8_t* grid, int64_t n_voxels, const uint8_t* emissive_entry,
-                                  uint32_t* counts, cudaStream_t st) {
-  const int64_t chunks = emissive_chunks(n_voxels);
+cudaError_t launch_emissive_count(const uint8_t* grid, const EmissiveVolume& V, const uint8_t* emissive_entry,
+                                  unsigned long long* counts, cudaStream_t st) {
+  const int64_t chunks = emissive_chunks(V.n);
   if (chunks <= 0) return cudaSuccess;
-  k_emissive_count<<<(unsigned)chunks, kEmThreads, 0, st>>>(grid, n_voxels, emissive_entry, counts);
+  k_emissive_count<<<(unsigned)chunks, kEmThreads, 0, st>>>(grid, V, emissive_entry, counts);
   k_emissive_offsets<<<1, kScanThreads, 0, st>>>(counts, chunks);
   return cudaGetLastError();
 }
 
-cudaError_t launch_emissive_write(const uint8_t* grid, int64_t n_voxels, const uint8_t* emissive_entry,
-                                  const uint32_t* offsets, int32_t* out, cudaStream_t st) {
-  const int64_t chunks = emissive_chunks(n_voxels);
-  if (chunks <= 0) return cudaSuccess;
-  k_emissive_write<<<(unsigned)chunks, kEmThreads, 0, st>>>(grid, n_voxels, emissive_entry, offsets, out);
+cudaError_t launch_emissive_write(const uint8_t* grid, const EmissiveVolume& V, const uint8_t* emissive_entry,
+                                  const unsigned long long* counts, int32_t* out, int64_t listed, int32_t* movers,
+                                  cudaStream_t st) {
+  const int64_t chunks = emissive_chunks(V.n);
+  if (chunks <= 0 || listed <= 0) return cudaSuccess;
+  k_emissive_write<<<(unsigned)chunks, kEmThreads, 0, st>>>(grid, V, emissive_entry, counts, chunks, out, movers);
+  if (movers) k_emissive_fill<<<(unsigned)((listed + 255) / 256), 256, 0, st>>>(movers, listed, out);
   return cudaGetLastError();
 }
 
@@ -243,104 +306,176 @@ __global__ void k_env_texels(const float* __restrict__ rgb, int64_t n, uint2* __
   lum[i] = (fr * 0.2126f + fg * 0.7152f) + fb * 0.0722f;
 }
 
-// 3x3 separable blur, clamp to edge (image.cpp:337-342), then the sin(theta)
-// weight and the max(0, .) of calculateImageIntegral (image.cpp:361-374).
-// Pass 0: horizontal into tmp; pass 1: vertical, * sin_theta[y] into func.
-__global__ void k_env_blur(const float* __restrict__ src, float* __restrict__ dst, int32_t w, int32_t h,
-                           int pass, const float* __restrict__ sin_theta) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (int64_t)w * h) return;
-  const int x = (int)(i % w), y = (int)(i / w);
-  float a, b, c;
-  if (pass == 0) {
-    const int xm = x > 0 ? x - 1 : 0, xp = x < w - 1 ? x + 1 : w - 1;
-    a = src[(int64_t)y * w + xm]; b = src[i]; c = src[(int64_t)y * w + xp];
-  } else {
-    const int ym = y > 0 ? y - 1 : 0, yp = y < h - 1 ? y + 1 : h - 1;
-    a = src[(int64_t)ym * w + x]; b = src[i]; c = src[(int64_t)yp * w + x];
-  }
-  float v = (VT_BLUR_SIDE * a + VT_BLUR_MID * b) + VT_BLUR_SIDE * c;
-  if (pass == 1) v = vtb::gmax(0.0f, v) * sin_theta[y];
-  dst[i] = v;
+// The sampled function of one texel: 3x3 separable blur of the luminance,
+// clamp to edge (image.cpp:337-342), then the max(0, .) and the sin(theta)
+// weight of calculateImageIntegral (image.cpp:361-374).
+__device__ __forceinline__ float blur_row(const float* __restrict__ lum, int32_t w, int x, int y) {
+  const float* r = lum + (int64_t)y * w;
+  const int xm = x > 0 ? x - 1 : 0, xp = x < w - 1 ? x + 1 : w - 1;
+  return (VT_BLUR_SIDE * r[xm] + VT_BLUR_MID * r[x]) + VT_BLUR_SIDE * r[xp];
+}
+__device__ __forceinline__ float env_function(const float* __restrict__ lum, int32_t w, int32_t h, int x, int y,
+                                              float sin_theta) {
+  const int ym = y > 0 ? y - 1 : 0, yp = y < h - 1 ? y + 1 : h - 1;
+  const float v = (VT_BLUR_SIDE * blur_row(lum, w, x, ym) + VT_BLUR_MID * blur_row(lum, w, x, y)) +
+                  VT_BLUR_SIDE * blur_row(lum, w, x, yp);
+  return vtb::gmax(0.0f, v) * sin_theta;
 }
 
-// Exclusive prefix sums in FP64 with a fixed association order, so that the
-// CPU restatement reproduces them exactly: consecutive chunks of 32 inputs
-// are summed left to right, chunk offsets are accumulated left to right, and
-// element prefix = chunk offset + in-chunk prefix.  out[0] = 0, out[n] = total.
-// One warp; offs holds ceil(n/32) doubles.
-template <typename T>
-__device__ void warp_chunked_prefix(const T* in, int n, double* out, double* offs) {
-  const int lane = threadIdx.x & 31;
-  const int chunks = (n + 31) / 32;
-  for (int c = lane; c < chunks; c += 32) {
-    double acc = 0.0;
-    const int end = min(n, (c + 1) * 32);
-    for (int j = c * 32; j < end; ++j) { acc = acc + (double)in[j]; out[j + 1] = acc; }
+// Prefix sums in FP64 with a fixed association order, so that the CPU
+// restatement reproduces them exactly: consecutive chunks of 32 inputs are
+// summed left to right, chunk offsets are accumulated left to right, and
+// element prefix = chunk offset + in-chunk prefix.  A block of kCdfThreads
+// threads takes kCdfTile inputs at a time: loaded coalesced into shared
+// memory (one double of padding per chunk), summed by a thread per chunk, the
+// offsets chained by thread 0 from one tile to the next.  What bounds it is
+// the length of the two chains, 32 additions and one per chunk; reading and
+// writing the chunks in global memory instead, a warp per row, cost a memory
+// round trip per addition (1024x512: 58 us for the rows, 19 for the marginal,
+// now 25 and 8.5, the 13 us of two blur passes folded in).
+constexpr int kCdfThreads = 128;
+constexpr int kCdfTile = 32 * kCdfThreads;
+__device__ __forceinline__ int cdf_at(int i) { return i + (i >> 5); }
+
+// Prefixes of in(0 .. n) in s (element i after input i, at cdf_at(i)), or past
+// the first tile in `pre` (element i after input i) as well; returns the total.
+template <class In>
+__device__ double block_chunked_prefix(const In& in, int n, double* s, double* s_off, double* __restrict__ pre) {
+  double carry = 0.0;   // offset of the tile's first chunk
+  const int tid = threadIdx.x;
+  for (int base = 0; base < n; base += kCdfTile) {
+    const int m = min(kCdfTile, n - base), chunks = (m + 31) / 32;
+    for (int i = threadIdx.x; i < m; i += kCdfThreads) s[cdf_at(i)] = (double)in(base + i);
+    __syncthreads();
+    if (tid < chunks) {
+      const int c0 = tid * 32, c1 = min(m, c0 + 32);
+      double* const sc = s + cdf_at(c0);   // a chunk lies contiguous
+      double acc = 0.0;
+      int i = 0;
+      for (; c0 + i + 8 <= c1; i += 8) {   // eight reads in flight ahead of the additions
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = sc[i + k];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          acc = acc + v[k];
+          sc[i + k] = acc;
+        }
+      }
+      for (; c0 + i < c1; ++i) {
+        acc = acc + sc[i];
+        sc[i] = acc;
+      }
+      s_off[tid] = acc;
+    }
+    __syncthreads();
+    if (tid < 32) {   // chunk totals -> offsets, 32 at a time from a warp's registers
+      double o = carry;
+      for (int c0 = 0; c0 < chunks; c0 += 32) {
+        const int c = c0 + tid;
+        const double t = c < chunks ? s_off[c] : 0.0;
+        double mine = 0.0;
+        for (int k = 0; k < 32 && c0 + k < chunks; ++k) {
+          const double tk = __shfl_sync(0xffffffffu, t, k);
+          if (tid == k) mine = o;
+          o = base + c0 + k == 0 ? tk : o + tk;
+        }
+        if (c < chunks) s_off[c] = mine;
+      }
+      if (tid == 0) s_off[kCdfThreads] = o;
+    }
+    __syncthreads();
+    carry = s_off[kCdfThreads];
+    const bool whole = n <= kCdfTile;
+    for (int i = threadIdx.x; i < m; i += kCdfThreads) {
+      const int c = i >> 5;
+      const double v = s[cdf_at(i)], p = base + c == 0 ? v : s_off[c] + v;
+      if (whole) s[cdf_at(i)] = p;
+      else pre[base + i] = p;
+    }
+    __syncthreads();
   }
-  __syncwarp();
-  if (lane == 0) {
-    out[0] = 0.0;
-    double o = 0.0;
-    offs[0] = 0.0;
-    for (int c = 1; c < chunks; ++c) { o = o + out[c * 32]; offs[c] = o; }
-  }
-  __syncwarp();
-  for (int c = lane; c < chunks; c += 32) {
-    if (c == 0) continue;
-    const double o = offs[c];
-    const int end = min(n, (c + 1) * 32);
-    for (int j = c * 32; j < end; ++j) out[j + 1] = o + out[j + 1];
-  }
-  __syncwarp();
+  return carry;
 }
 
-// One warp per row (image.cpp:212-247): FP64 prefixes of the row function,
-// normalised conditional CDF (uniform if the row is black), row integral =
-// row sum / width.
-__global__ void k_cdf_rows(const float* __restrict__ func, int32_t w, int32_t h, double* __restrict__ pre_all,
-                           float* __restrict__ cdf_u, double* __restrict__ row_int) {
-  extern __shared__ double s_offs[];
+// (float)(a / b) for 0 <= a <= b, b normal: a product with the reciprocal is
+// within two units of the double quotient, so both round to the same float
+// unless the product lies that close to the middle of two floats or below
+// the normal floats; those few divide.
+__device__ __forceinline__ float quotient(double a, double b, double rcp) {
+  const double q = a * rcp;
+  const uint32_t low = (uint32_t)__double_as_longlong(q) & 0x1fffffffu;   // bits below a float's
+  if (q >= 1.2e-38 && low - 0x0ffffff8u > 16u) return (float)q;
+  return (float)(a / b);
+}
+
+// One block per row (image.cpp:212-247): the row of the sampled function
+// (kEnv: from the luminance; otherwise given), its FP64 prefixes, normalised
+// conditional CDF (uniform if the row is black), row integral = row sum / width.
+template <bool kEnv>
+__global__ void __launch_bounds__(kCdfThreads) k_cdf_rows(const float* __restrict__ f, int32_t w, int32_t h,
+                                                          const float* __restrict__ sin_theta,
+                                                          double* __restrict__ pre_all, float* __restrict__ cdf_u,
+                                                          double* __restrict__ row_int) {
+  __shared__ double s[kCdfTile + kCdfThreads];
+  __shared__ double s_off[kCdfThreads + 1];
   const int row = blockIdx.x;
-  const int lane = threadIdx.x & 31;
-  if (row >= h) return;
   double* pre = pre_all + (int64_t)row * (w + 1);
-  warp_chunked_prefix(func + (int64_t)row * w, w, pre, s_offs);
-  const double total = pre[w];
+  double total;
+  if constexpr (kEnv) {
+    const float st = sin_theta[row];
+    total = block_chunked_prefix([&](int x) { return env_function(f, w, h, x, row, st); }, w, s, s_off, pre);
+  } else {
+    total = block_chunked_prefix([&](int x) { return f[(int64_t)row * w + x]; }, w, s, s_off, pre);
+  }
   float* out = cdf_u + (int64_t)row * (w + 1);
-  for (int x = lane; x <= w; x += 32) {
-    if (total > 0.0) out[x] = (float)(pre[x] / total);
+  if (threadIdx.x == 0) {   // one thread's divisions: FP64 is scarce
+    s_off[0] = 1.0 / total;
+    row_int[row] = total / (double)w;
+  }
+  __syncthreads();
+  const double rcp = s_off[0];
+  const bool whole = w <= kCdfTile;
+  for (int x = threadIdx.x; x <= w; x += kCdfThreads) {
+    if (total > 0.0) out[x] = x == 0 ? 0.0f : quotient(whole ? s[cdf_at(x - 1)] : pre[x - 1], total, rcp);
     else out[x] = (float)x / (float)w;
   }
-  if (lane == 0) row_int[row] = total / (double)w;
 }
 
 // Marginal CDF over the row integrals (image.cpp:251-280) and the radiance
-// integral 2 pi^2 * mean(f) (image.cpp:381-386).  One warp.
-__global__ void k_cdf_marginal(const double* __restrict__ row_int, int32_t h, double* __restrict__ pre,
-                               float* __restrict__ cdf_v, float* integral) {
-  extern __shared__ double s_offs[];
-  const int lane = threadIdx.x & 31;
-  warp_chunked_prefix(row_int, h, pre, s_offs);
-  const double total = pre[h];
-  for (int y = lane; y <= h; y += 32) {
-    if (total > 0.0) cdf_v[y] = (float)(pre[y] / total);
+// integral 2 pi^2 * mean(f) (image.cpp:381-386).  One block.
+__global__ void __launch_bounds__(kCdfThreads) k_cdf_marginal(const double* __restrict__ row_int, int32_t h,
+                                                              double* __restrict__ pre, float* __restrict__ cdf_v,
+                                                              float* integral) {
+  __shared__ double s[kCdfTile + kCdfThreads];
+  __shared__ double s_off[kCdfThreads + 1];
+  const double total = block_chunked_prefix([&](int y) { return row_int[y]; }, h, s, s_off, pre);
+  if (threadIdx.x == 0) s_off[0] = 1.0 / total;
+  __syncthreads();
+  const double rcp = s_off[0];
+  const bool whole = h <= kCdfTile;
+  for (int y = threadIdx.x; y <= h; y += kCdfThreads) {
+    if (total > 0.0) cdf_v[y] = y == 0 ? 0.0f : quotient(whole ? s[cdf_at(y - 1)] : pre[y - 1], total, rcp);
     else cdf_v[y] = (float)y / (float)h;
   }
-  if (lane == 0 && integral) {
+  if (threadIdx.x == 0 && integral) {
     *integral = (float)((total / (double)h) * (2.0 * 3.14159265358979323846 * 3.14159265358979323846));
   }
 }
 
-cudaError_t launch_cdf(const float* func, int32_t w, int32_t h, const EnvScratch& S, float* cdf_u,
-                       float* cdf_v, float* integral, cudaStream_t st) {
-  const size_t sm_rows = sizeof(double) * (size_t)((w + 31) / 32);
-  const size_t sm_marg = sizeof(double) * (size_t)((h + 31) / 32);
-  k_cdf_rows<<<h, 32, sm_rows, st>>>(func, w, h, S.row_pre, cdf_u, S.row_int);
+template <bool kEnv>
+static cudaError_t cdf(const float* f, int32_t w, int32_t h, const EnvScratch& S, float* cdf_u, float* cdf_v,
+                       float* integral, cudaStream_t st) {
+  k_cdf_rows<kEnv><<<h, kCdfThreads, 0, st>>>(f, w, h, S.sin_theta, S.row_pre, cdf_u, S.row_int);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_cdf_marginal<<<1, 32, sm_marg, st>>>(S.row_int, h, S.marg_pre, cdf_v, integral);
+  k_cdf_marginal<<<1, kCdfThreads, 0, st>>>(S.row_int, h, S.marg_pre, cdf_v, integral);
   return cudaGetLastError();
+}
+
+cudaError_t launch_cdf(const float* func, int32_t w, int32_t h, const EnvScratch& S, float* cdf_u,
+                       float* cdf_v, float* integral, cudaStream_t st) {
+  return cdf<false>(func, w, h, S, cdf_u, cdf_v, integral, st);
 }
 
 // The CDF image of a shrunk environment (image.cpp:308-320): each output
@@ -378,13 +513,11 @@ cudaError_t launch_env_build(const float* rgb, int32_t w, int32_t h, int32_t cw,
   const int64_t n = (int64_t)w * h;
   k_env_texels<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(rgb, n, texels, S.lum, bad);
   const int64_t m = (int64_t)cw * ch;
-  const unsigned blocks = (unsigned)((m + 255) / 256);
-  if (cw != w || ch != h) k_env_shrink_lum<<<blocks, 256, 0, st>>>(texels, w, h, cw, ch, S.lum);
-  k_env_blur<<<blocks, 256, 0, st>>>(S.lum, S.tmp, cw, ch, 0, S.sin_theta);
-  k_env_blur<<<blocks, 256, 0, st>>>(S.tmp, S.func, cw, ch, 1, S.sin_theta);
+  if (cw != w || ch != h)
+    k_env_shrink_lum<<<(unsigned)((m + 255) / 256), 256, 0, st>>>(texels, w, h, cw, ch, S.lum);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  return launch_cdf(S.func, cw, ch, S, cdf_u, cdf_v, integral, st);
+  return cdf<true>(S.lum, cw, ch, S, cdf_u, cdf_v, integral, st);
 }
 
 // --------------------------------------------------------------- voxelizer
