@@ -76,7 +76,8 @@ VT_API int vt_diag_cdf_from_function(vt_context* ctx, const float* func, int32_t
  * and trace_blocks_per_sm < 0 keep their value):
  * path_slots paths in flight per launch (default 2M), trace_blocks_per_sm
  * resident blocks of the DDA kernel (0: occupancy limit, the default),
- * trace_steps DDA steps between ray-pool refills (4, 8, 16 or 32; default 16),
+ * trace_steps DDA steps between ray-pool refills (4, 8, 16 or 32; by default
+ * 16, 8 where a volume has free cubes),
  * max_items samples per launch (sample-buffer entries, default 2^28). */
 VT_API int vt_diag_set_tuning(vt_context* ctx, int64_t path_slots, int32_t trace_blocks_per_sm,
                               int32_t trace_steps, int64_t max_items);

@@ -272,6 +272,7 @@ vt_scene::~vt_scene() {
   if (!ctx) return;
   ctx->release(grid);
   ctx->release(bricks);
+  ctx->release(runs.load());
   ctx->release(palette);
   ctx->release(emissive);
 }
@@ -1162,13 +1163,15 @@ int vt::build_frame(vt_job* j) {
   int rc = vt_camera_compute_uniforms(&j->cam, j->w, j->h, &U);
   if (rc != VT_OK) return rc;
   memcpy(F.viewport, U.viewport, sizeof(F.viewport));
-  memcpy(F.proj, U.proj, sizeof(F.proj));
+  F.proj_zz = U.proj[10];
+  F.proj_zw = U.proj[11];
+  F.proj_wz = U.proj[14];
   memcpy(F.inv_proj, U.inv_proj, sizeof(F.inv_proj));
   memcpy(F.inv_mv, U.inv_model_view, sizeof(F.inv_mv));
   F.frag_z = 0.5f * j->cam.near_distance + 0.5f;
   // screen_to_eye_persp's depth terms at frag_z, in its operation order
   F.persp_ndc_z = ((2.0f * F.frag_z - 0.0f) - 1.0f) / (1.0f - 0.0f);
-  F.persp_cw = F.proj[11] / (F.persp_ndc_z - (F.proj[10] / F.proj[14]));
+  F.persp_cw = F.proj_zw / (F.persp_ndc_z - (F.proj_zz / F.proj_wz));
   F.lens_radius = j->cam.lens_radius;
   F.focal_distance = j->cam.focal_distance;
   F.lens_model = j->cam.lens_model;
@@ -1203,6 +1206,7 @@ int vt::build_frame(vt_job* j) {
   JobDev& D = j->dev;
   D.grid = s->grid;
   D.bricks = s->bricks;
+  D.runs = s->runs.load();
   D.palette = s->palette;
   D.emissive = s->emissive;
   D.env_texels = j->env ? j->env->texels : nullptr;
@@ -1314,6 +1318,61 @@ extern "C" int vt_job_set_integrator(vt_job* j, int32_t integrator) {
   return vt_job_reset(j);   // the reference restarts the accumulation on a switch (renderer.cpp:678-683)
 }
 
+// The free cubes of a scene about to be rendered, built on the rendering
+// context's stream and kept with the scene.  They only speed the DDA up: none
+// for other brick shapes, for scenes of a context with a memory budget (the
+// budget is the caller's to spend), where memory is short, or where too little
+// of the volume is open for a leap to pay: the line lies at a tenth of the
+// bricks starting an empty cube of four bricks a side.  Measured, without ->
+// with free cubes: 1024^3 shell (0.90 of the bricks) 1024^2 x 16 spp 19.9 ->
+// 11.3 ms; 256^3 noise (0.15) 1024^2 x 256 spp 123.4 -> 117.1 ms; 64^3 spheres
+// (0.08) 564 -> 575 us; 128^3 noise (0.006) 472 -> 497 us.
+constexpr double kOpenFraction = 0.1;
+static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
+  vt_scene* s = const_cast<vt_scene*>(scene);
+  std::lock_guard<std::mutex> g(s->runs_mu);
+  if (s->runs_tried || s->bsh[0] != 2 || s->bsh[1] != 2 || s->bsh[2] != 2) return VT_OK;
+  s->runs_tried = true;
+  if (s->ctx->budget || !s->ctx->free_cubes) return VT_OK;
+  const int32_t bx = s->bdim[0], by = s->bdim[1], bz = s->bdim[2];
+  void* scratch = nullptr;
+  if (s->ctx->alloc(&scratch, free_cube_scratch_bytes(bx, by, bz)) != VT_OK) return VT_OK;
+  uint32_t* d_open = nullptr;
+  uint32_t open[32];   // pageable: the read has completed when the copy returns
+  cudaError_t e = launch_free_cubes_open(s->bricks, bx, by, bz, scratch, &d_open, ctx->sm_count, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(open, d_open, sizeof(open), cudaMemcpyDeviceToHost, ctx->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  double n_open = 0.0;
+  for (uint32_t v : open) n_open += v;
+  const size_t bytes = sizeof(unsigned long long) * (size_t)(bx + 2) * (by + 2) * (bz + 2);
+  void* runs = nullptr;
+  if (e == cudaSuccess && n_open >= kOpenFraction * bx * by * bz && s->ctx->alloc(&runs, bytes) == VT_OK) {
+    e = launch_free_cubes(bx, by, bz, scratch, (unsigned long long*)runs, ctx->stream);
+    // other streams may render the scene next, and the scratch goes back
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  }
+  s->ctx->release(scratch);
+  if (e != cudaSuccess) {
+    s->ctx->release(runs);
+    return cuda_fail(e, "free cubes");
+  }
+  if (!runs) return VT_OK;
+  s->bytes += bytes;
+  s->runs.store((unsigned long long*)runs);
+  s->generation += 1;   // jobs rebuild their frames before their next pass
+  return VT_OK;
+}
+
+// DDA steps between refills of a launch: the caller's choice, or 16, 8 where a
+// volume has free cubes (256^3 noise 121.9 -> 117.1 ms; 16 without them 123.4,
+// 8 127 ms).
+static int launch_trace_steps(const vt_context* ctx, const std::vector<Grid>& grids) {
+  if (ctx->trace_steps > 0) return ctx->trace_steps;
+  for (const Grid& g : grids)
+    if (g.runs) return 8;
+  return 16;
+}
+
 // Launch `passes` samples per pixel for a set of jobs with the selected kernel.
 int vt::refresh_job(vt_job* j) {
   if (j->scene && j->scene_generation != j->scene->generation) return build_frame(j);
@@ -1325,7 +1384,8 @@ int vt::render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32
   vt::Range nvtx_range("vt.render");
   cudaSetDevice(ctx->device);
   for (int32_t i = 0; i < n; ++i) {
-    const int rc = refresh_job(jobs[i]);
+    int rc = count ? VT_OK : ensure_free_cubes(ctx, jobs[i]->scene);
+    if (rc == VT_OK) rc = refresh_job(jobs[i]);
     if (rc != VT_OK) return rc;
   }
   if (count) VT_CUDA(cudaMemsetAsync(ctx->d_counters, 0, sizeof(unsigned long long) * C_NUM, ctx->stream), "counters");
@@ -1505,7 +1565,7 @@ static int block_launch(vt_context* ctx, const std::vector<JobEntry>& entries, c
   P.next_item = ctx->d_queue + 2;
   P.n_items = (unsigned long long)items;
   P.sbuf = ctx->sbuf;
-  P.trace_steps = ctx->trace_steps;
+  P.trace_steps = launch_trace_steps(ctx, grids);
   // a path ends within max_bounces + 2 rounds of its start: the wavefront's
   // bound, for a block that takes every sample
   P.max_rounds = (int32_t)std::min<int64_t>(4 * (items / slots + 2) * ((int64_t)max_b + 2) + 16, 0x7fffffff);
@@ -1593,6 +1653,7 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
                               : (ctx->trace_blocks_per_sm > 0 ? ctx->trace_blocks_per_sm : ctx->trace_occupancy);
   if (lanes > 1 && blocks_per_sm <= 0 && ctx->trace_blocks_per_sm <= 0) bps = std::max(1, bps * 2 / 3);
   const int trace_blocks = ctx->sm_count * bps;
+  const int trace_steps = launch_trace_steps(ctx, grids);
   // Eight rounds of every lane: per round and lane its counters cleared,
   // shade + hit + regen, trace.  The other lanes' streams fork from the
   // first and join it again, so the group is one unit of work on `st` (one
@@ -1608,7 +1669,7 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
         e = cudaMemsetAsync(P[l].ctl + ctl_index(par, 0), 0, CTL_PER_PARITY * kCtlStride * sizeof(uint32_t),
                             lane_st[l]);
         if (e == cudaSuccess) e = launch_wf_shade(P[l], par, ctx->sm_count * 8, count, lane_st[l], T);
-        if (e == cudaSuccess) e = launch_wf_trace(P[l], par, trace_blocks, ctx->trace_steps, count, lane_st[l], T);
+        if (e == cudaSuccess) e = launch_wf_trace(P[l], par, trace_blocks, trace_steps, count, lane_st[l], T);
       }
     }
     for (int l = 1; l < lanes && e == cudaSuccess; ++l) {
@@ -1722,7 +1783,7 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
       e.n_pixels = (int64_t)jobs[i]->w * jobs[i]->h;
       items += e.n_pixels * p;
       entries.push_back(e);
-      grids.push_back(make_grid(jobs[i]->frame, jobs[i]->dev.bricks));
+      grids.push_back(make_grid(jobs[i]->frame, jobs[i]->dev.bricks, jobs[i]->dev.runs));
       done[i] += p;
     }
     if (items >= ((int64_t)1 << 32)) return fail(VT_EINVAL, "more than 2^32 samples in one launch");
@@ -1842,6 +1903,9 @@ extern "C" int vt_scene_set_voxel(vt_scene* s, int32_t x, int32_t y, int32_t z, 
   const int64_t idx = (int64_t)x + (int64_t)s->res[0] * ((int64_t)y + (int64_t)s->res[1] * z);
   VT_CUDA(launch_set_voxel(s->grid, s->bricks, s->res[0], s->res[1], s->bdim[0], s->bdim[1], scene_shape(s), x, y,
                            z, (uint8_t)entry, ctx->stream), "voxel edit");
+  if (entry && s->runs.load())
+    VT_CUDA(launch_free_cubes_edit(s->runs.load(), s->bdim[0], s->bdim[1], s->bdim[2], x >> 2, y >> 2, z >> 2,
+                                   ctx->stream), "voxel edit");
   int rc = VT_OK;
   if (s->flags & VT_SCENE_AUTO_EMISSIVE) {
     rc = scene_emissive(ctx, s, nullptr, 0, s->flags);          // rediscover from the palette
@@ -2112,6 +2176,13 @@ extern "C" int vt_scene_set_brick_shape(vt_scene* s, int32_t sx, int32_t sy, int
   const int64_t old_nb = (int64_t)(s->bdim[0] + 2) * (s->bdim[1] + 2) * (s->bdim[2] + 2);
   ctx->release(s->bricks);
   s->bricks = bricks;
+  {   // the free cubes are those of the old shape
+    std::lock_guard<std::mutex> g(s->runs_mu);
+    unsigned long long* runs = s->runs.exchange(nullptr);
+    if (runs) s->bytes -= sizeof(unsigned long long) * (uint64_t)old_nb;
+    ctx->release(runs);
+    s->runs_tried = false;
+  }
   for (int i = 0; i < 3; ++i) s->bdim[i] = bdim[i];
   s->bytes = s->bytes - sizeof(unsigned long long) * (uint64_t)old_nb + sizeof(unsigned long long) * (uint64_t)nb;
   s->generation++;   // jobs on this scene rebuild their frames before their next pass

@@ -26,7 +26,9 @@ constexpr size_t round256(size_t x) { return (x + 255) & ~(size_t)255; }
 constexpr size_t kSlotBytes = kWfSlotBytes;
 constexpr size_t kCtlOff = 0;
 constexpr size_t kJobsOff = kCtlOff + round256(kCtlBytes);
-constexpr size_t kGridsOff = kJobsOff + round256(sizeof(JobEntry) * VT_FIXED_MAX_JOBS);
+constexpr size_t kJobsBytes = 9472;   // what the public size of the array holds for the job table
+static_assert(sizeof(JobEntry) * VT_FIXED_MAX_JOBS <= kJobsBytes, "the job table outgrew its part");
+constexpr size_t kGridsOff = kJobsOff + kJobsBytes;
 constexpr size_t kSlotsOff = kGridsOff + round256(sizeof(Grid) * VT_FIXED_MAX_JOBS);
 constexpr size_t kSamplesOff = kSlotsOff + round256(kSlotBytes * (size_t)VT_FIXED_MAX_PATH_SLOTS);
 constexpr size_t kTotal = kSamplesOff + sizeof(float4) * (size_t)VT_FIXED_MAX_SAMPLES;
@@ -85,7 +87,7 @@ static int drain(vt_context* ctx, int rc) {
   return rc;
 }
 
-static Grid fixed_grid(const vt_job* j) { return make_grid(j->frame, j->dev.bricks); }
+static Grid fixed_grid(const vt_job* j) { return make_grid(j->frame, j->dev.bricks, j->dev.runs); }
 
 // One wavefront launch over entries[0..n) with `items` samples in total.
 static int fixed_launch(vt_context* ctx, char* base, const JobEntry* entries, const Grid* grids, int n,
@@ -124,6 +126,9 @@ static int fixed_launch(vt_context* ctx, char* base, const JobEntry* entries, co
   if (ctx->trace_occupancy <= 0) ctx->trace_occupancy = std::max(1, wf_trace_blocks_per_sm());
   const int bps = ctx->trace_blocks_per_sm > 0 ? ctx->trace_blocks_per_sm : ctx->trace_occupancy;
   const int trace_blocks = ctx->sm_count * bps;
+  bool runs = false;
+  for (int i = 0; i < n; ++i) runs = runs || grids[i].runs != nullptr;
+  const int trace_steps = ctx->trace_steps > 0 ? ctx->trace_steps : (runs ? 8 : 16);
   // the bound of the wavefront launch's loop: a path ends within
   // max_bounces + 2 rounds of its start
   int32_t max_b = 0;
@@ -137,7 +142,7 @@ static int fixed_launch(vt_context* ctx, char* base, const JobEntry* entries, co
     if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed round counters"));
     e = launch_wf_shade(P, par, ctx->sm_count * 8, false, st);
     if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed wavefront shade"));
-    e = launch_wf_trace(P, par, trace_blocks, ctx->trace_steps, false, st);
+    e = launch_wf_trace(P, par, trace_blocks, trace_steps, false, st);
     if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed wavefront trace"));
     ctx->launches += 4;
     if ((iter & 7) == 7) {

@@ -11,6 +11,12 @@
 //                                   every side has all bits set, as do voxels of
 //                                   the last bricks beyond the volume, so that a
 //                                   ray leaving the volume stops on a set bit
+//   runs     uint64[...] (same bricks, 4x4x4 shape only; built at the first render,
+//                                   may be absent)  byte o of a brick's word, o =
+//                                   (dx > 0) | (dy > 0) << 1 | (dz > 0) << 2: the level
+//                                   (free_cube_side) of an empty cube of bricks that starts
+//                                   with this one and extends towards octant o (0: the brick
+//                                   holds an occupied voxel); a lower bound of the largest
 //   palette  uint4[n_palette]       one 16-byte record per material: eight IEEE
 //                                   halves {type, emission rgb, albedo rgb, roughness}
 //   emissive int32[n_emissive]      linear voxel indices sampled by NEE
@@ -27,6 +33,14 @@
 
 namespace vt {
 
+// Sides of the free cubes (JobDev::runs) in bricks, by level: 0, 1, 2, 3, 4,
+// 6, 8, 12, 16, five bits each.
+constexpr int kMaxFreeCube = 16;
+__host__ __device__ __forceinline__ uint32_t free_cube_side(uint32_t level) {
+  constexpr uint64_t sides = 0ull | 1ull << 5 | 2ull << 10 | 3ull << 15 | 4ull << 20 | 6ull << 25 | 8ull << 30 |
+                             12ull << 35 | 16ull << 40;
+  return (uint32_t)(sides >> (5u * level)) & 31u;
+}
 constexpr int kNoiseW = 1024;   // reference noise texture size (renderer.cpp:749-758)
 constexpr int kNoiseH = 1024;
 constexpr float kInfinity = 99999999.0f;  // focalDistance.vs:43
@@ -44,7 +58,7 @@ struct Frame {
   int32_t bsh[3];            // log2 of a brick's extent along x, y, z (sum 6)
   float viewport[4];
   float frag_z;              // gl_FragCoord.z of the full-screen quad drawn at z = near
-  float proj[16];            // row-major, as uploaded with transpose = GL_TRUE
+  float proj_zz, proj_zw, proj_wz;   // entries 10, 11 and 14 of the row-major projection
   float inv_proj[16];
   float inv_mv[16];
   float lens_radius;
@@ -129,6 +143,7 @@ struct Grid {
   int32_t mx, my, mz;        // brick extents - 1
   int32_t n_words;           // words of the padded brick array (bounds of the checked build)
   const unsigned long long* bricks;   // brick (0,0,0) of the padded array
+  const unsigned long long* runs;     // the same brick's free cubes, null without them
 };
 
 // Bit of voxel (x, y, z) in its brick word (brick shape shifts and masks).
@@ -137,7 +152,8 @@ __host__ __device__ __forceinline__ int brick_bit(int x, int y, int z, int shx, 
 }
 
 // The DDA's view of a volume (frame uniforms + the job's brick array).
-__host__ __device__ __forceinline__ Grid make_grid(const Frame& F, const unsigned long long* bricks) {
+__host__ __device__ __forceinline__ Grid make_grid(const Frame& F, const unsigned long long* bricks,
+                                                        const unsigned long long* runs) {
   Grid g;
   g.rx = F.res[0]; g.ry = F.res[1]; g.rz = F.res[2];
   g.bx = F.bdim[0] + 2; g.bxy = (F.bdim[0] + 2) * (F.bdim[1] + 2);
@@ -151,6 +167,7 @@ __host__ __device__ __forceinline__ Grid make_grid(const Frame& F, const unsigne
   const long long nw = (long long)g.bxy * (F.bdim[2] + 2);
   g.n_words = nw < 0x7fffffffLL ? (int32_t)nw : 0x7fffffff;
   g.bricks = bricks + 1 + g.bx + g.bxy;   // brick (0,0,0) inside the border
+  g.runs = runs ? runs + 1 + g.bx + g.bxy : nullptr;
   return g;
 }
 
@@ -158,6 +175,7 @@ __host__ __device__ __forceinline__ Grid make_grid(const Frame& F, const unsigne
 struct JobDev {
   const uint8_t* grid;
   const unsigned long long* bricks;
+  const unsigned long long* runs;   // null without them
   const uint4* palette;
   const int32_t* emissive;
   const uint2* env_texels;

@@ -164,6 +164,18 @@ cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t 
 cudaError_t launch_build_bricks(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
                                 unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, const BrickShape& sh,
                                 unsigned long long* max_entry, cudaStream_t st);
+// Free cubes of a volume's 4x4x4 bricks (vt_internal.h), in two launches over
+// the same scratch (free_cube_scratch_bytes bytes of device memory): the first
+// leaves at *open 32 counts whose sum is the number of bricks that start an
+// empty cube of four bricks a side, the second writes a word per padded brick.
+size_t free_cube_scratch_bytes(int32_t bx, int32_t by, int32_t bz);
+cudaError_t launch_free_cubes_open(const unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, void* scratch,
+                                   uint32_t** open, int sm_count, cudaStream_t st);
+cudaError_t launch_free_cubes(int32_t bx, int32_t by, int32_t bz, void* scratch, unsigned long long* runs,
+                              cudaStream_t st);
+// After brick (x, y, z) became occupied.
+cudaError_t launch_free_cubes_edit(unsigned long long* runs, int32_t bx, int32_t by, int32_t bz, int32_t x, int32_t y,
+                                   int32_t z, cudaStream_t st);
 // A volume as the emissive passes see it.
 struct EmissiveVolume {
   int32_t rx, ry, rz;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -44,7 +45,7 @@ struct vt_context {
   int64_t max_items = 1 << 28;   // samples per launch (sample buffer entries)
   int trace_blocks_per_sm = 0;   // 0 = occupancy limit
   int trace_occupancy = 0;       // occupancy limit of the DDA kernel (cached)
-  int trace_steps = 16;          // DDA steps between refills of the trace kernel
+  int trace_steps = 0;           // DDA steps between refills (0: by the launch's volumes)
   int trace_chunk = 64;          // queue records per warp atomic of the trace kernel (at most)
   int refill_min = 0;            // early refill of a trace warp below this many stepping lanes (0 = off)
   int trace_form = 0;            // DDA kernel form: 0 per-lane segment set-up, 1 pooled set-up
@@ -70,6 +71,7 @@ struct vt_context {
   int alloc(void** ptr, size_t bytes);
   void release(void* ptr);
   uint64_t trim(uint64_t keep);           // free cached blocks down to `keep` bytes; returns bytes freed
+  bool free_cubes = true;       // scenes of this context may hold free cubes
   bool caching = true;
   std::multimap<size_t, void*> cache;     // size -> block
   uint64_t cached = 0;
@@ -93,7 +95,11 @@ struct vt_scene {
   int64_t n_emissive = 0;
   uint64_t bytes = 0;
   uint32_t flags = 0;            // creation flags (emissive list policy for edits)
-  uint64_t generation = 0;       // bumped by edits that move device buffers
+  std::atomic<uint64_t> generation{0};   // bumped by edits that move device buffers
+  // free cubes (vt_internal.h), built by the first render of the scene
+  std::atomic<unsigned long long*> runs{nullptr};
+  bool runs_tried = false;       // built, or not to be had (under runs_mu)
+  std::mutex runs_mu;
   std::vector<vt_material> host_palette;
   // the reference's flat material table and the record offset of each
   // palette entry in it (-1: the entry has no record there)

@@ -70,6 +70,211 @@ __global__ void __launch_bounds__(32 * kBrickRows) k_build_bricks(const uint8_t*
     atomicMax(max_entry, (unsigned long long)top);
 }
 
+// ------------------------------------------------------------- free cubes
+// Per 4x4x4 brick and octant, the side in bricks of an empty cube of bricks
+// that starts with the brick and extends towards the octant: 1, 2, 3, 4, 6, 8,
+// 12 or 16, the largest of these that is empty.  The DDA crosses such a cube
+// in one leap (dda_leap).
+//
+// A bitmap per side over the padded brick rows, 32 bricks a word, bit set:
+// the cube of that side from the brick towards +x, +y, +z is empty (bricks
+// beyond the padded array count as occupied).  The cube towards another
+// octant is the same cube seen from its other end, so eight bitmaps serve the
+// eight octants.  Three passes of word operations and one that turns bits
+// into bytes: 1024^3 (17 M bricks) takes about as long as reading the bricks
+// and writing the bytes.
+constexpr int kCubeSides = 8;
+__device__ constexpr int kCubeSide[kCubeSides] = {1, 2, 3, 4, 6, 8, 12, 16};   // free_cube_side of 1 .. 8
+static int64_t cube_words(int32_t bx) { return ((int64_t)bx + 2 + 31) / 32; }
+size_t free_cube_scratch_bytes(int32_t bx, int32_t by, int32_t bz) {
+  return sizeof(uint32_t) * (kCubeSides * (size_t)(cube_words(bx) * (by + 2) * (bz + 2)) + 32);
+}
+
+// Side 1, one warp per word: bit i set if brick 32 w + i of the row is empty.
+// (A bitmap has fewer than 2^31 words: 32-bit indices and divisions.)
+__global__ void k_cubes_1(const unsigned long long* __restrict__ bricks, int32_t px, uint32_t n, uint32_t words,
+                          uint32_t* __restrict__ e1) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  for (uint32_t i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
+    const uint32_t r = i / words;
+    const int x = (int)(i - r * words) * 32 + lane;
+    const uint32_t w = __ballot_sync(0xffffffffu, x < px && bricks[(int64_t)r * px + x] == 0ull);
+    if (lane == 0) e1[i] = w;
+  }
+}
+
+// 64 bricks of row (y, z) from word w on; none beyond the array.
+__device__ __forceinline__ unsigned long long cube_bits(const uint32_t* __restrict__ e, int w, int y, int z, int32_t words,
+                                                        int32_t py, int32_t pz) {
+  if (y >= py || z >= pz) return 0ull;
+  const uint32_t* r = e + ((int64_t)z * py + y) * words + w;
+  return (unsigned long long)r[0] | (w + 1 < words ? (unsigned long long)r[1] << 32 : 0ull);
+}
+
+// Sides 2, 3 and 4 from side 1, and behind the bitmaps the number of bricks
+// that start a cube of side 4 (in 32 parts); sides 6, 8, 12 and 16 from sides 3 and 4.
+__global__ void k_cubes_small(uint32_t* __restrict__ e, int32_t words, int32_t py, int32_t pz) {
+  const int64_t n = (int64_t)words * py * pz;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t row = i / (uint32_t)words;
+  const int w = (int)(i - row * words), z = (int)(row / (uint32_t)py), y = (int)(row - (uint32_t)z * py);
+  uint32_t c2 = ~0u, c3 = ~0u, c4 = ~0u;
+  for (int dz = 0; dz < 4; ++dz)
+    for (int dy = 0; dy < 4; ++dy) {
+      const unsigned long long r = cube_bits(e, w, y + dy, z + dz, words, py, pz);
+      const unsigned long long x2 = r & (r >> 1);
+      if (dz < 2 && dy < 2) c2 &= (uint32_t)x2;
+      if (dz < 3 && dy < 3) c3 &= (uint32_t)(x2 & (r >> 2));
+      c4 &= (uint32_t)(x2 & (x2 >> 2));
+    }
+  e[n + i] = c2;
+  e[2 * n + i] = c3;
+  e[3 * n + i] = c4;
+  const uint32_t open = (uint32_t)__popc(c4);
+  if (open) atomicAdd(&e[kCubeSides * n + (threadIdx.x & 31)], open);
+}
+__global__ void k_cubes_large(uint32_t* __restrict__ e, int32_t words, int32_t py, int32_t pz) {
+  const int64_t n = (int64_t)words * py * pz;
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t row = i / (uint32_t)words;
+  const int w = (int)(i - row * words), z = (int)(row / (uint32_t)py), y = (int)(row - (uint32_t)z * py);
+  uint32_t c6 = ~0u, c8 = ~0u, c12 = ~0u, c16 = ~0u;
+  for (int dz = 0; dz < 2; ++dz)
+    for (int dy = 0; dy < 2; ++dy) {
+      const unsigned long long r = cube_bits(e + 2 * n, w, y + 3 * dy, z + 3 * dz, words, py, pz);
+      c6 &= (uint32_t)(r & (r >> 3));
+    }
+  for (int dz = 0; dz < 4; ++dz)
+    for (int dy = 0; dy < 4; ++dy) {
+      const unsigned long long r = cube_bits(e + 3 * n, w, y + 4 * dy, z + 4 * dz, words, py, pz);
+      const unsigned long long x8 = r & (r >> 4);
+      if (dz < 2 && dy < 2) c8 &= (uint32_t)x8;
+      if (dz < 3 && dy < 3) c12 &= (uint32_t)(x8 & (r >> 8));
+      c16 &= (uint32_t)(x8 & (x8 >> 8));
+    }
+  e[4 * n + i] = c6;
+  e[5 * n + i] = c8;
+  e[6 * n + i] = c12;
+  e[7 * n + i] = c16;
+}
+
+// One warp per word: lane 4 o + q gathers octant o of bricks 8 q .. 8 q + 7;
+// the bytes change places through shared memory into a word per brick.
+// A warp takes kCubeRun words in a row: its octants read eight rows of each
+// bitmap, and a sector holds eight words of one (a word per warp in turn
+// fetched every sector eight times: 200 us for 1024^3).
+constexpr int kCubeWarps = 4;
+constexpr uint32_t kCubeRun = 8;
+__global__ void __launch_bounds__(32 * kCubeWarps) k_cubes_bytes(const uint32_t* __restrict__ e, int32_t words,
+                                                                 int32_t px, int32_t py, int32_t pz,
+                                                                 unsigned long long* __restrict__ runs) {
+  __shared__ __align__(8) uint8_t s[kCubeWarps][32][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int o = lane >> 2, q = lane & 3;
+  const uint32_t n = (uint32_t)words * py * pz;
+  const uint32_t first = (blockIdx.x * kCubeWarps + warp) * kCubeRun, last = min(n, first + kCubeRun);
+  const uint32_t down = ((o & 2) ? 0u : (uint32_t)words) + ((o & 4) ? 0u : (uint32_t)words * py);
+  const uint32_t row = first / (uint32_t)words;
+  int w = (int)(first - row * words), z = (int)(row / (uint32_t)py), y = (int)(row - (uint32_t)z * py);
+  for (uint32_t i = first; i < last; ++i) {
+    // the cube's lowest row lies (side - 1) rows and slices down where the
+    // octant's y, z point down: in the array if side - 1 is at most `low`
+    const int low = min((o & 2) ? kMaxFreeCube : y, (o & 4) ? kMaxFreeCube : z);
+    uint32_t c[kCubeSides];
+#pragma unroll
+    for (int k = 0; k < kCubeSides; ++k) {   // every read is issued before any is used
+      const int off = kCubeSide[k] - 1;
+      const uint32_t* r = e + (size_t)k * n + (i - (uint32_t)off * down);
+      const bool in = off <= low;
+      const uint32_t cur = in ? r[0] : 0u, prev = in && !(o & 1) && w > 0 ? r[-1] : 0u;
+      c[k] = (o & 1) ? cur : __funnelshift_l(prev, cur, off);   // and from its lowest brick
+    }
+    // levels passed, 0 to 8, in four bit planes: each level implies the ones before it
+    const uint32_t b0 = (c[0] & ~c[1]) | (c[2] & ~c[3]) | (c[4] & ~c[5]) | (c[6] & ~c[7]);
+    const uint32_t b1 = (c[1] & ~c[3]) | (c[5] & ~c[7]);
+    const uint32_t b2 = c[3] & ~c[7], b3 = c[7];
+    uint32_t lo = 0u, hi = 0u;   // a byte per brick
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t v = (k == 0 ? b0 : k == 1 ? b1 : k == 2 ? b2 : b3) >> (8 * q);
+      lo |= (((v & 15u) * 0x00204081u) & 0x01010101u) << k;
+      hi |= ((((v >> 4) & 15u) * 0x00204081u) & 0x01010101u) << k;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s[warp][8 * q + j][o] = (uint8_t)(lo >> (8 * j));
+      s[warp][8 * q + 4 + j][o] = (uint8_t)(hi >> (8 * j));
+    }
+    __syncwarp();
+    const int x = 32 * w + lane;
+    if (x < px) runs[((int64_t)z * py + y) * px + x] = *(const unsigned long long*)s[warp][lane];
+    __syncwarp();
+    if (++w == words) {
+      w = 0;
+      if (++y == py) { y = 0; ++z; }
+    }
+  }
+}
+
+cudaError_t launch_free_cubes_open(const unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, void* scratch,
+                                   uint32_t** open, int sm_count, cudaStream_t st) {
+  const int32_t words = (int32_t)cube_words(bx), py = by + 2, pz = bz + 2;
+  const int64_t n = (int64_t)words * py * pz;
+  uint32_t* e = (uint32_t*)scratch;
+  *open = e + kCubeSides * n;
+  const cudaError_t m = cudaMemsetAsync(*open, 0, 32 * sizeof(uint32_t), st);
+  if (m != cudaSuccess) return m;
+  k_cubes_1<<<(unsigned)std::min<int64_t>((n + 7) / 8, (int64_t)sm_count * 64), 256, 0, st>>>(bricks, bx + 2,
+                                                                                             (uint32_t)n, words, e);
+  k_cubes_small<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(e, words, py, pz);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_free_cubes(int32_t bx, int32_t by, int32_t bz, void* scratch, unsigned long long* runs,
+                              cudaStream_t st) {
+  const int32_t words = (int32_t)cube_words(bx), py = by + 2, pz = bz + 2;
+  const int64_t n = (int64_t)words * py * pz, per_block = kCubeWarps * kCubeRun;
+  uint32_t* e = (uint32_t*)scratch;
+  k_cubes_large<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(e, words, py, pz);
+  k_cubes_bytes<<<(unsigned)((n + per_block - 1) / per_block), 32 * kCubeWarps, 0, st>>>(e, words, bx + 2, py, pz, runs);
+  return cudaGetLastError();
+}
+
+// Free cubes around a brick that became occupied: a cube that holds it ends
+// before it.  One thread per brick within reach; a brick that became empty
+// leaves them as they are, still lower bounds.
+constexpr int kReach = 2 * kMaxFreeCube - 1;
+__global__ void k_cubes_edit(unsigned long long* runs, int32_t px, int32_t py, int32_t pz, int32_t x, int32_t y,
+                             int32_t z) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kReach * kReach * kReach) return;
+  const int ox = i % kReach - (kMaxFreeCube - 1), oy = (i / kReach) % kReach - (kMaxFreeCube - 1),
+            oz = i / (kReach * kReach) - (kMaxFreeCube - 1);
+  const int vx = x - ox, vy = y - oy, vz = z - oz;   // the edited brick lies (ox, oy, oz) from this one
+  if (vx < 0 || vy < 0 || vz < 0 || vx >= px || vy >= py || vz >= pz) return;
+  const uint32_t d = (uint32_t)max(abs(ox), max(abs(oy), abs(oz)));
+  unsigned long long* at = runs + ((int64_t)vx + (int64_t)px * ((int64_t)vy + (int64_t)py * vz));
+  unsigned long long w = *at;
+  for (int o = 0; o < 8; ++o) {
+    const bool towards = ((o & 1) ? ox >= 0 : ox <= 0) && ((o & 2) ? oy >= 0 : oy <= 0) && ((o & 4) ? oz >= 0 : oz <= 0);
+    uint32_t level = (uint32_t)(w >> (8 * o)) & 0xffu;
+    if (!towards || free_cube_side(level) <= d) continue;
+    while (free_cube_side(level) > d) --level;
+    w = (w & ~(0xffull << (8 * o))) | ((unsigned long long)level << (8 * o));
+  }
+  *at = w;
+}
+
+cudaError_t launch_free_cubes_edit(unsigned long long* runs, int32_t bx, int32_t by, int32_t bz, int32_t x, int32_t y,
+                                   int32_t z, cudaStream_t st) {
+  const int n = kReach * kReach * kReach;
+  k_cubes_edit<<<(n + 127) / 128, 128, 0, st>>>(runs, bx + 2, by + 2, bz + 2, x + 1, y + 1, z + 1);
+  return cudaGetLastError();
+}
+
 // One voxel edit: its grid entry and its bit in the padded brick grid.
 __global__ void k_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t rx, int32_t ry, int32_t bx, int32_t by,
                             const BrickShape sh, int32_t x, int32_t y, int32_t z, uint8_t entry) {

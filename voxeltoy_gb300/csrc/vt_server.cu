@@ -330,6 +330,7 @@ extern "C" int vt_server_create(vt_context* ctx, const vt_server_opts* opts, vt_
   U.sm_count = ctx->sm_count;
   U.log_fn = ctx->log_fn;
   U.log_user = ctx->log_user;
+  U.free_cubes = s->opts.hbm_budget_bytes == 0;   // they would count against an admission budget
   e = cudaStreamCreateWithFlags(&U.stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { release_context(&L); delete s; return cuda_fail(e, "server upload stream"); }
   rc = U.alloc((void**)&U.d_counters, sizeof(unsigned long long) * C_NUM);

@@ -253,7 +253,7 @@ VT_D v3 world_to_local(v3 w, const Basis& b) {
 }
 
 // -------------------------------------------------------------------- dda
-VT_D Grid grid_of(const Frame& F, const JobDev& J) { return make_grid(F, J.bricks); }
+VT_D Grid grid_of(const Frame& F, const JobDev& J) { return make_grid(F, J.bricks, J.runs); }
 
 struct Dda {
   int32_t x, y, z;
@@ -450,6 +450,72 @@ done:
 
 VT_D bool bricks_444(const Grid& g) { return g.shx == 2 && g.shy == 2 && g.shz == 2; }
 
+// Level of the free cube at a running segment's position towards its octant.
+// The position is in the volume or one voxel outside, where the padded bricks
+// hold none.
+VT_D int dda_room(const Grid& g, const Dda& s) {
+  const int b = (s.x >> 2) + g.bx * (s.y >> 2) + g.bxy * (s.z >> 2);
+  const int o = (s.sx > 0 ? 1 : 0) | (s.sy > 0 ? 2 : 0) | (s.sz > 0 ? 4 : 0);
+  const long long w = (long long)b + 1 + g.bx + g.bxy;   // index in the padded array
+  return chk(w >= 0 && w < g.n_words, CHK_BRICK) ? (int)__ldg((const uint8_t*)(g.runs + b) + o) : 0;
+}
+
+// Crossings of one axis at or before T: d becomes the first one after T, and
+// their number is returned.  d is the next crossing, and the ones after it are
+// the running sums f(j + 1) = fl(f(j) + a) that the DDA loop forms.  Within a
+// binade those sums rise by one constant: the distance of two of them is a
+// rounded to a multiple of the binade's ulp, and where a lies halfway between
+// two multiples, ties to even settle after the first sum.  T lies below the
+// end of the binade of f(1), so from f(2) on (that sum settled) every f(j) up
+// to T is f(2) + (j - 2) i, exactly, with i = f(3) - f(2).  The quotient by an
+// approximate reciprocal is off by at most one, which the compares mend, and
+// the last sum is formed as the loop forms it.  `most` only bounds the result
+// for increments that are not numbers of this kind.
+VT_D int dda_crossings(float& d, float a, float T, float most) {
+  const float f1 = d + a, f2 = f1 + a;
+  const float i = (f2 + a) - f2;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(i));
+  float m = fmaxf(fminf(floorf((T - f2) * r), most), 0.0f);
+  float last = __fmaf_rn(m, i, f2);                 // f(m + 2), exact
+  if (last > T) {
+    m = m - 1.0f;
+    last = __fmaf_rn(m, i, f2);
+  }
+  float next = last + a;
+  if (next <= T) {
+    m = m + 1.0f;
+    next = next + a;
+  }
+  const bool c0 = d <= T, c1 = f1 <= T, c2 = f2 <= T;
+  const int k = c2 ? (int)m + 3 : (c1 ? 2 : (c0 ? 1 : 0));
+  d = c2 ? next : (c1 ? f2 : (c0 ? f1 : d));
+  return k;
+}
+
+// Moves a running segment through the free cube at its position, of level 2
+// or more, in one go: to the state that the DDA loop has after every crossing
+// up to a time T before the first one that leaves the cube.  T: a crossing
+// that leaves is a sum of at most 64 increments, each rounded by 2^-24 of its
+// value at most, so it lies above 0.9998 of the unrounded sum; and no sum up
+// to T may leave the binade of its axis's next-but-one crossing.
+VT_D void dda_leap(Dda& s, int room) {
+  const int reach = 4 * (int)free_cube_side((uint32_t)room) - 4;
+  const float nx = (float)(reach + (s.sx > 0 ? 3 - (s.x & 3) : (s.x & 3)));   // crossings that stay inside
+  const float ny = (float)(reach + (s.sy > 0 ? 3 - (s.y & 3) : (s.y & 3)));
+  const float nz = (float)(reach + (s.sz > 0 ? 3 - (s.z & 3) : (s.z & 3)));
+  const float tx = __uint_as_float((__float_as_uint(s.dx + s.ax) & 0x7f800000u) + 0x00800000u);   // binade ends
+  const float ty = __uint_as_float((__float_as_uint(s.dy + s.ay) & 0x7f800000u) + 0x00800000u);
+  const float tz = __uint_as_float((__float_as_uint(s.dz + s.az) & 0x7f800000u) + 0x00800000u);
+  const float leave = fminf(__fmaf_rn(nx, s.ax, s.dx), fminf(__fmaf_rn(ny, s.ay, s.dy), __fmaf_rn(nz, s.az, s.dz)));
+  const float T = fminf(leave, fminf(tx, fminf(ty, tz))) * 0.9998f;
+  const int kx = dda_crossings(s.dx, s.ax, T, nx), ky = dda_crossings(s.dy, s.ay, T, ny),
+            kz = dda_crossings(s.dz, s.az, T, nz);
+  s.x += s.sx * kx;
+  s.y += s.sy * ky;
+  s.z += s.sz * kz;
+}
+
 // One whole segment that dda_begin set up, in the per-lane kernels: the
 // counted loop, or without event counts the 4x4x4 loop where the grid's bricks
 // have that shape.
@@ -462,7 +528,13 @@ VT_D void dda_finish(const Grid& g, Dda& s, Cnt<kCount>& cnt) {
     dda_steps<kCount, false, true>(g, s, 0x7fffffff, cnt, 0);
   } else {
     dda_end_stuck(g, s);
-    if (s.state == DDA_RUNNING) dda_steps_444<false>(g, s, 1 << 30, 0);
+    while (s.state == DDA_RUNNING) {
+      if (g.runs) {
+        const int room = dda_room(g, s);
+        if (room >= 2) dda_leap(s, room);
+      }
+      dda_steps_444<false>(g, s, g.runs ? 8 : 1 << 30, 0);
+    }
   }
 }
 
@@ -737,7 +809,7 @@ VT_D float4 screen_to_eye_persp(const Frame& F, v3 w) {
     cw = F.persp_cw;
   } else {
     ndc.z = ((2.0f * w.z - 0.0f) - 1.0f) / (1.0f - 0.0f);
-    cw = F.proj[11] / (ndc.z - (F.proj[10] / F.proj[14]));
+    cw = F.proj_zw / (ndc.z - (F.proj_zz / F.proj_wz));
   }
   return mul4(F.inv_proj, make_float4(ndc.x * cw, ndc.y * cw, ndc.z * cw, cw));
 }
