@@ -1325,7 +1325,7 @@ extern "C" int vt_job_set_integrator(vt_job* j, int32_t integrator) {
 // of the volume is open for a leap to pay: the line lies at a tenth of the
 // bricks starting an empty cube of four bricks a side.  Measured, without ->
 // with free cubes: 1024^3 shell (0.90 of the bricks) 1024^2 x 16 spp 19.9 ->
-// 11.3 ms; 256^3 noise (0.15) 1024^2 x 256 spp 123.4 -> 117.1 ms; 64^3 spheres
+// 9.3 ms; 256^3 noise (0.15) 1024^2 x 256 spp 123.4 -> 114.2 ms; 64^3 spheres
 // (0.08) 564 -> 575 us; 128^3 noise (0.006) 472 -> 497 us.
 constexpr double kOpenFraction = 0.1;
 static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
@@ -1364,8 +1364,8 @@ static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
 }
 
 // DDA steps between refills of a launch: the caller's choice, or 16, 8 where a
-// volume has free cubes (256^3 noise 121.9 -> 117.1 ms; 16 without them 123.4,
-// 8 127 ms).
+// volume has free cubes (256^3 noise 119.1 -> 114.2 ms, 4 119.0; without them 16
+// 123.4, 8 127 ms).
 static int launch_trace_steps(const vt_context* ctx, const std::vector<Grid>& grids) {
   if (ctx->trace_steps > 0) return ctx->trace_steps;
   for (const Grid& g : grids)

@@ -492,16 +492,17 @@ __global__ void __launch_bounds__(128, RegenBlocks<Tab>::value) k_wf_regen(const
   flush_counters(cnt, P.counters);
 }
 
-// Before a warp's step loop: its segments that stand in a large enough free
-// cube cross it in one leap (dda_leap, some 110 instructions for the whole
-// warp against 33 a step), when at least kLeapLanes of them do.  All lanes of
-// the warp must call it.
-constexpr int kLeapLanes = 12;
-template <class GridRef>
-__device__ __forceinline__ void warp_leap(const GridRef& g, Dda& s, bool have) {
-  int room = 0;
-  if (have && g.runs) room = dda_room(g, s);
-  if (__popc(__ballot_sync(0xffffffffu, room >= 2)) >= kLeapLanes && room >= 2) dda_leap(s, room);
+// Before a warp's step loop: segments that stand in a large enough free cube
+// cross it in one leap (dda_leap, some 110 instructions for the warp, however
+// few of its lanes take it, against 33 a step).  Asking for 4, 8 or 12 such
+// lanes first measured slower: a 1024^3 shell 10.5, 11.2, 11.3 ms against 9.3,
+// 256^3 noise 1-2%.
+// A second leap where the first one ends in another cube: shell 8.8 ms, noise
+// 118.8 against 114.2 ms.
+__device__ __forceinline__ void leap(const Grid& g, Dda& s) {
+  if (!g.runs) return;
+  const int room = dda_room(g, s);
+  if (room >= 2) dda_leap(s, room);
 }
 
 // The grid record of a lane's current segment: a register copy, or with one
@@ -592,8 +593,8 @@ __global__ void __launch_bounds__(256, TraceBlocks<Tab>::value) k_wf_trace(const
       }
       if (!__any_sync(FULL, have) && !more && pool >= pool_end) break;
     }
-    if constexpr (!kCount && k444) warp_leap(gh.get(T), s, have);
     if (have) {
+      if constexpr (!kCount && k444) leap(gh.get(T), s);
       if constexpr (!kCount && k444) dda_steps_444<kVote>(gh.get(T), s, kTraceSteps, P.refill_min);
       else dda_steps<kCount, kVote, k444>(gh.get(T), s, kTraceSteps, cnt, P.refill_min);
       if (s.state != DDA_RUNNING) {
@@ -957,8 +958,8 @@ __global__ void __launch_bounds__(kBlockThreads, kBlocksPerSm) k_paths_block(con
           }
         }
         if (!more && !__any_sync(FULL, have)) break;
-        if constexpr (k444) warp_leap(gh.get(T), s, have);
         if (have) {
+          if constexpr (k444) leap(gh.get(T), s);
           if constexpr (k444) dda_steps_444<false>(gh.get(T), s, P.trace_steps, 0);
           else dda_steps<false, false, false>(gh.get(T), s, P.trace_steps, cnt, 0);
           if (s.state != DDA_RUNNING) {
