@@ -1400,7 +1400,7 @@ int vt::render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32
       continue;
     }
     for (int k = 0; k < passes[i]; ++k)
-      VT_CUDA(launch_plain(j->frame, j->dev, j->samples + k, 1, count ? ctx->d_counters : nullptr, ctx->stream),
+      VT_CUDA(launch_plain(j->frame, j->dev, j->samples + k, 1, ctx->sm_count, count ? ctx->d_counters : nullptr, ctx->stream),
               "plain render");
     ctx->launches += (uint64_t)passes[i];
   }
@@ -1482,7 +1482,8 @@ constexpr int64_t kBlockItems = 3 << 20;
 // the accumulation; a single pass of one job accumulates as it goes.
 static int paths_launch(vt_context* ctx, const std::vector<JobEntry>& entries, int64_t items) {
   if (entries.size() == 1 && entries[0].passes == 1) {
-    VT_CUDA(launch_plain(entries[0].F, entries[0].J, entries[0].sample_base, 1, nullptr, ctx->stream), "pass");
+    VT_CUDA(launch_plain(entries[0].F, entries[0].J, entries[0].sample_base, 1, ctx->sm_count, nullptr,
+                         ctx->stream), "pass");
     ctx->launches += 1;
     return VT_OK;
   }
@@ -1500,7 +1501,7 @@ static int paths_launch(vt_context* ctx, const std::vector<JobEntry>& entries, i
   P.n_jobs = (int32_t)entries.size();
   P.n_items = (unsigned long long)items;
   P.sbuf = ctx->sbuf;
-  VT_CUDA(launch_paths(P, ctx->stream, entries.size() <= (size_t)kWfParamJobs ? &table : nullptr), "samples");
+  VT_CUDA(launch_paths(P, ctx->sm_count, ctx->stream, entries.size() <= (size_t)kWfParamJobs ? &table : nullptr), "samples");
   long long max_pixels = 0;
   for (const JobEntry& e : entries) max_pixels = std::max<long long>(max_pixels, e.n_pixels);
   VT_CUDA(launch_wf_accumulate(ctx->d_jobs, (int)entries.size(), max_pixels, ctx->sbuf, ctx->stream), "accumulate");

@@ -196,7 +196,7 @@ extern "C" int vt_render_batch_fixed(vt_context* ctx, vt_job* const* jobs, int32
   for (int i = 0; i < n_jobs; ++i) {
     if (jobs[i]->integrator == VT_INTEGRATOR_PATH_TRACER) continue;
     for (int32_t k = 0; k < np[i]; ++k) {
-      e = launch_plain(jobs[i]->frame, jobs[i]->dev, jobs[i]->samples + k, 1, nullptr, ctx->stream);
+      e = launch_plain(jobs[i]->frame, jobs[i]->dev, jobs[i]->samples + k, 1, ctx->sm_count, nullptr, ctx->stream);
       if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed edit-mode pass"));
     }
     ctx->launches += (uint64_t)np[i];

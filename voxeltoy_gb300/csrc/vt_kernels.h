@@ -20,7 +20,7 @@ struct JobEntry {
 };
 
 // ---- render (vt_render.cu)
-cudaError_t launch_plain(const Frame& F, const JobDev& J, int sample_base, int passes,
+cudaError_t launch_plain(const Frame& F, const JobDev& J, int sample_base, int passes, int sm_count,
                          unsigned long long* counters, cudaStream_t st);
 cudaError_t launch_diag(const Frame& F, const JobDev& J, int sample, float4* out, HitRecord* hits,
                         unsigned long long* counters, cudaStream_t st);
@@ -135,7 +135,7 @@ struct BlockParams {
 cudaError_t launch_paths_block(const BlockParams& P, int blocks, cudaStream_t st, const WfJobTable* T = nullptr);
 // Every sample of a launch by a thread of its own (jobs, n_jobs, n_items and
 // sbuf of P), outputs into sbuf as the wavefront's.
-cudaError_t launch_paths(const WfParams& P, cudaStream_t st, const WfJobTable* T = nullptr);
+cudaError_t launch_paths(const WfParams& P, int sm_count, cudaStream_t st, const WfJobTable* T = nullptr);
 cudaError_t launch_wf_accumulate(const JobEntry* jobs, int n_jobs, long long max_pixels, const float4* sbuf,
                                  cudaStream_t st);
 int wf_trace_blocks_per_sm();

@@ -32,16 +32,29 @@ __device__ __forceinline__ void flush_counters(Cnt<kCount>& cnt, unsigned long l
   }
 }
 
+// Samples a warp of the thread-per-sample kernels takes, 8, 16 or 32: the
+// fewest that leave about one wave of warps (16 an SM are resident).  A warp
+// runs the union of its lanes' paths, so a launch that leaves warps free
+// spreads its samples over more of them, down to 8 (160x120 samples of 64^3
+// spheres 142 us at 32 a warp, 125 at 16, 118 at 8; 240x180 143, 129, 132;
+// 256x192 of 128^3 noise 218, 232, 319).
+int samples_per_warp(int64_t n, int sm_count) {
+  int per = 8;
+  while (per < 32 && (n + per - 1) / per > 18 * (int64_t)sm_count) per *= 2;
+  return per;
+}
+
 // ------------------------------------------------------------------ plain
 template <bool kCount>
 __global__ void __launch_bounds__(128) k_plain(const Frame F, const JobDev J, int sample_base, int passes,
-                                               unsigned long long* counters) {
+                                               int per_warp, unsigned long long* counters) {
   Cnt<kCount> cnt;
 #pragma unroll
   for (int i = 0; i < C_NUM; ++i) cnt.c[i] = 0;
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int idx = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane;
   const int n = F.width * F.height;
-  if (idx < n) {
+  if (lane < per_warp && idx < n) {
     const int px = idx % F.width, py = idx / F.width;
     float4 sum = J.sum[idx], comp = J.comp[idx];
     for (int k = 0; k < passes; ++k) {
@@ -54,13 +67,14 @@ __global__ void __launch_bounds__(128) k_plain(const Frame F, const JobDev J, in
   flush_counters(cnt, counters);
 }
 
-cudaError_t launch_plain(const Frame& F, const JobDev& J, int sample_base, int passes,
+cudaError_t launch_plain(const Frame& F, const JobDev& J, int sample_base, int passes, int sm_count,
                          unsigned long long* counters, cudaStream_t st) {
   const int n = F.width * F.height;
   const int threads = 128;
-  const int blocks = (n + threads - 1) / threads;
-  if (counters) k_plain<true><<<blocks, threads, 0, st>>>(F, J, sample_base, passes, counters);
-  else k_plain<false><<<blocks, threads, 0, st>>>(F, J, sample_base, passes, nullptr);
+  const int per_warp = samples_per_warp(n, sm_count);
+  const int warps = (n + per_warp - 1) / per_warp, blocks = (warps + threads / 32 - 1) / (threads / 32);
+  if (counters) k_plain<true><<<blocks, threads, 0, st>>>(F, J, sample_base, passes, per_warp, counters);
+  else k_plain<false><<<blocks, threads, 0, st>>>(F, J, sample_base, passes, per_warp, nullptr);
   return cudaGetLastError();
 }
 
@@ -990,9 +1004,11 @@ cudaError_t launch_paths_block(const BlockParams& P, int blocks, cudaStream_t st
 // Launches of few samples, where only the longest path's time counts: one
 // thread carries a whole sample from the camera to its output.
 template <class Tab>
-__global__ void __launch_bounds__(128) k_paths(const WfParams P, const __grid_constant__ Tab T) {
-  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P.n_items) return;
+__global__ void __launch_bounds__(128) k_paths(const WfParams P, const __grid_constant__ Tab T, int per_warp) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long i =
+      (unsigned long long)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per_warp + lane;
+  if (lane >= per_warp || i >= P.n_items) return;
   const JobEntry& E = job_entry(P, T, (uint32_t)job_of(P, T, i));
   const uint32_t r = (uint32_t)(i - (unsigned long long)E.tile_begin);
   const uint32_t pass = udiv(r, E.F.m_pixels);
@@ -1043,11 +1059,12 @@ cudaError_t launch_wf_shade(const WfParams& P, int par, int persist_blocks, bool
   return cudaGetLastError();
 }
 
-cudaError_t launch_paths(const WfParams& P, cudaStream_t st, const WfJobTable* T) {
-  const unsigned blocks = (unsigned)((P.n_items + 127) / 128);
-  if (T && P.n_jobs == 1) k_paths<<<blocks, 128, 0, st>>>(P, one_job(*T));
-  else if (T && P.n_jobs <= kWfParamJobs) k_paths<<<blocks, 128, 0, st>>>(P, *T);
-  else k_paths<<<blocks, 128, 0, st>>>(P, WfNoTable{0});
+cudaError_t launch_paths(const WfParams& P, int sm_count, cudaStream_t st, const WfJobTable* T) {
+  const int per_warp = samples_per_warp((int64_t)P.n_items, sm_count);
+  const unsigned blocks = (unsigned)((P.n_items + 4 * per_warp - 1) / (4 * per_warp));   // four warps
+  if (T && P.n_jobs == 1) k_paths<<<blocks, 128, 0, st>>>(P, one_job(*T), per_warp);
+  else if (T && P.n_jobs <= kWfParamJobs) k_paths<<<blocks, 128, 0, st>>>(P, *T, per_warp);
+  else k_paths<<<blocks, 128, 0, st>>>(P, WfNoTable{0}, per_warp);
   return cudaGetLastError();
 }
 
