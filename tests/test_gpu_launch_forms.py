@@ -12,7 +12,8 @@ from voxeltoy_gb300 import Context, Job
 
 pytestmark = pytest.mark.gpu
 
-PATHS, BLOCK = 1 << 17, 3 << 20      # kPathsItems, kBlockItems
+PATHS = 1 << 17             # kPathsItems
+BLOCK = (16 << 20) // 10    # kBlockWork over the rounds of eight bounces: 1677721
 
 
 @pytest.fixture(scope="module")
@@ -54,7 +55,7 @@ def config2(w, h, edge=24, seed=11):
 @pytest.mark.parametrize("w,h,passes", [
     (1, 1, 1), (1, 1, 33), (31, 1, 2), (33, 7, 5),             # a thread per sample
     (512, 256, 1), (512, 257, 1), (256, 128, 4),               # PATHS, past it
-    (1024, 1024, 3), (1024, 1025, 3), (701, 499, 3),           # BLOCK, past it, between
+    (1024, 819, 2), (1024, 820, 2), (701, 499, 3),             # BLOCK, past it, between
 ])
 def test_forms_agree_at_their_limits(fctx, w, h, passes):
     compare(fctx, [config2(w, h)], passes)

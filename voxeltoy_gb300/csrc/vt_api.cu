@@ -1473,10 +1473,16 @@ static int jobs_upload(vt_context* ctx, const std::vector<JobEntry>& entries) {
 }
 
 // Samples per launch up to which each gets a thread of its own (k_paths), and
-// up to which block wavefronts carry them (k_paths_block, with the times on
-// both sides of either line).
+// samples times rounds (max_bounces + 2) up to which block wavefronts carry
+// them (k_paths_block): a round costs the wavefront its kernels' launches, and
+// the block form loses with every sample's share of a round.  Block against
+// wavefront, us: eight bounces, 1.57 M samples of 128^3 noise 1301 / 1301, 2.1 M
+// 1591 / 1489, 1.05 M and 2.1 M of 256^3 noise 1286 / 1374 and 2008 / 1831, 2.1 M
+// of a 1024^3 shell 2163 / 2253; five bounces, 2.1 M and 3.1 M of a 203x117x89
+// volume 694 / 896 and 905 / 1034; four bounces, 1.57 M, 2.1 M and 3.1 M of 64^3
+// spheres 740 / 779, 904 / 890 and 1230 / 1165.
 constexpr int64_t kPathsItems = 1 << 17;
-constexpr int64_t kBlockItems = 3 << 20;
+constexpr int64_t kBlockWork = 16 << 20;
 
 // A launch of at most kPathsItems samples: one kernel over the samples, then
 // the accumulation; a single pass of one job accumulates as it goes.
@@ -1655,21 +1661,31 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
   if (lanes > 1 && blocks_per_sm <= 0 && ctx->trace_blocks_per_sm <= 0) bps = std::max(1, bps * 2 / 3);
   const int trace_blocks = ctx->sm_count * bps;
   const int trace_steps = launch_trace_steps(ctx, grids);
-  // Eight rounds of every lane: per round and lane its counters cleared,
-  // shade + hit + regen, trace.  The other lanes' streams fork from the
-  // first and join it again, so the group is one unit of work on `st` (one
-  // CUDA graph when graphs are on); within it the lanes run free of each
-  // other.
+  // Where every sample has a slot, all paths start in the first round and end
+  // within max_bounces + 2: one group of that many rounds, launched directly
+  // (the capture of a graph that runs once costs more than it saves).
+  // Otherwise groups of eight rounds, replayed as a graph.  With groups of
+  // eight in both, each with five nodes a round (the counters cleared by a
+  // node of their own), 4.2 M samples of 128^3 noise with eight bounces took
+  // 2.71 ms, now 2.31; 8.4 M of 256^3 noise 5.21 and 4.62.
+  int32_t max_b = 0;
+  for (const JobEntry& e : entries) max_b = std::max(max_b, e.F.max_bounces);
+  const int64_t lane_items = (items + lanes - 1) / lanes;
+  const bool one_fill = lane_items <= (int64_t)lane_slots && max_b + 2 <= 16;
+  const int rounds = one_fill ? (max_b + 3) & ~1 : 8;   // even: the last has parity 1
+  const bool use_graphs = ctx->use_graphs && !one_fill;
+  // A group of rounds of every lane: per round and lane shade + hit + regen,
+  // trace.  The other lanes' streams fork from the first and join it again,
+  // so the group is one unit of work on `st` (one CUDA graph when graphs are
+  // on); within it the lanes run free of each other.
   auto group = [&]() -> cudaError_t {
     cudaError_t e = cudaSuccess;
     if (lanes > 1) e = cudaEventRecord(ctx->lane_ready, st);
     for (int l = 1; l < lanes && e == cudaSuccess; ++l) e = cudaStreamWaitEvent(lane_st[l], ctx->lane_ready, 0);
-    for (int r = 0; r < 8 && e == cudaSuccess; ++r) {
+    for (int r = 0; r < rounds && e == cudaSuccess; ++r) {
       const int par = r & 1;
       for (int l = 0; l < lanes && e == cudaSuccess; ++l) {
-        e = cudaMemsetAsync(P[l].ctl + ctl_index(par, 0), 0, CTL_PER_PARITY * kCtlStride * sizeof(uint32_t),
-                            lane_st[l]);
-        if (e == cudaSuccess) e = launch_wf_shade(P[l], par, ctx->sm_count * 8, count, lane_st[l], T);
+        e = launch_wf_shade(P[l], par, ctx->sm_count * 8, count, lane_st[l], T);
         if (e == cudaSuccess) e = launch_wf_trace(P[l], par, trace_blocks, trace_steps, count, lane_st[l], T);
       }
     }
@@ -1679,7 +1695,7 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
     }
     return e;
   };
-  if (ctx->use_graphs) {
+  if (use_graphs) {
     cudaGraph_t graph = nullptr;
     VT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture rounds");
     const cudaError_t ce = group();
@@ -1716,21 +1732,18 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
   // within (items / slots + 2) * (max_bounces + 2) rounds.  Four times that
   // bounds the loop, so a fault in the kernels' bookkeeping ends the call
   // with an error instead of looping.
-  int32_t max_b = 0;
-  for (const JobEntry& e : entries) max_b = std::max(max_b, e.F.max_bounces);
-  const int64_t lane_items = (items + lanes - 1) / lanes;
   const int64_t drain_rounds = (lane_items / (int64_t)lane_slots + 2) * ((int64_t)max_b + 2);
-  const int64_t max_groups = 4 * (drain_rounds + 7) / 8 + 4;
+  const int64_t max_groups = 4 * (drain_rounds + 7) / rounds + 4;
   for (int64_t group_n = 0;; ++group_n) {
     if (group_n >= max_groups)
-      return fail(VT_EDEVICE, "wavefront did not drain within %lld rounds", (long long)(8 * max_groups));
-    vt::Range rounds_range("vt.rounds");   // eight rounds of every lane, then the live-count check
-    if (ctx->use_graphs) {
+      return fail(VT_EDEVICE, "wavefront did not drain within %lld rounds", (long long)(rounds * max_groups));
+    vt::Range rounds_range("vt.rounds");   // a group of rounds of every lane, then the live-count check
+    if (use_graphs) {
       VT_CUDA(cudaGraphLaunch(ctx->rounds_exec, st), "wavefront rounds");
     } else {
       VT_CUDA(group(), "wavefront rounds");
     }
-    ctx->launches += (uint64_t)lanes * 8 * 4;
+    ctx->launches += (uint64_t)lanes * rounds * 4;
     for (int l = 0; l < lanes; ++l)
       VT_CUDA(cudaMemcpyAsync(ctx->h_live + l, P[l].ctl + ctl_index(1, CTL_NEXT_N), sizeof(uint32_t),
                               cudaMemcpyDeviceToHost, st),
@@ -1788,8 +1801,10 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
       done[i] += p;
     }
     if (items >= ((int64_t)1 << 32)) return fail(VT_EINVAL, "more than 2^32 samples in one launch");
-    int rc = by_size && items <= kPathsItems   ? paths_launch(ctx, entries, items)
-             : by_size && items <= kBlockItems ? block_launch(ctx, entries, grids, items)
+    int64_t max_b = 0;
+    for (const JobEntry& e : entries) max_b = std::max<int64_t>(max_b, e.F.max_bounces);
+    int rc = by_size && items <= kPathsItems ? paths_launch(ctx, entries, items)
+             : by_size && items * (max_b + 2) <= kBlockWork ? block_launch(ctx, entries, grids, items)
                                              : wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
     if (rc != VT_OK) return rc;
   }

@@ -138,8 +138,6 @@ static int fixed_launch(vt_context* ctx, char* base, const JobEntry* entries, co
     if (iter >= max_rounds) return drain(ctx, fail(VT_EDEVICE, "wavefront did not drain within %lld rounds",
                                                    (long long)max_rounds));
     const int par = (int)(iter & 1);
-    e = cudaMemsetAsync(ctl + ctl_index(par, 0), 0, CTL_PER_PARITY * kCtlStride * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed round counters"));
     e = launch_wf_shade(P, par, ctx->sm_count * 8, false, st);
     if (e != cudaSuccess) return drain(ctx, cuda_fail(e, "fixed wavefront shade"));
     e = launch_wf_trace(P, par, trace_blocks, trace_steps, false, st);

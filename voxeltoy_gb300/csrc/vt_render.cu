@@ -442,6 +442,9 @@ __global__ void __launch_bounds__(128, RegenBlocks<Tab>::value) k_wf_regen(const
     P.ctl[ctl_index(par, CTL_NEXT_N)] = n_hits + m;
     P.ctl[ctl_index(par, CTL_REGEN_N)] = m;
   }
+  // the next round's counters: this round's shading, which read the stream
+  // length among them, is done
+  if (blockIdx.x == 0 && threadIdx.x < CTL_PER_PARITY) P.ctl[ctl_index(par ^ 1, (int)threadIdx.x)] = 0u;
   const WfState& dst = P.x[par ^ 1];
   float4* const q = P.queue[par];
   Cnt<kCount> cnt;
@@ -734,21 +737,18 @@ __global__ void __launch_bounds__(256, 4) k_wf_trace_pool(const WfParams P, cons
 // one counter until none is left.  Blocks never wait for one another, so a
 // launch is one kernel.
 //
-// A wavefront launch costs some 0.45 ms before its first path (0.85 ms with
-// eight bounces: two groups of rounds): kernels of a few microseconds, five a
-// round and lane, and the capture of their graph.  Here a round costs its
-// block three barriers.  Per sample the block form is the slower one: all
-// four parts run at the registers of the largest (64, 1024 threads an SM), and
-// a block of a thousand paths ends every DDA part waiting for its longest
-// segments.  Measured (us, thread per sample / block / wavefront):
-//   19 k samples of 64^3 spheres          142 /  170 /  435
-//   262 k of 128^3 noise, 8 bounces       610 /  460 /  975
-//   1.05 M of 64^3 spheres                805 /  561 /  744
-//   2.1 M of a 203x117x89 noise volume   1477 /  688 /  928
-//   3.1 M of 128^3 noise, 256^3 noise       - / 2219, 2916 / 2272, 3025
-//   3.1 M of a 1024^3 shell                 - / 6230 / 5817
-//   4.2 M of 128^3 noise                    - / 2930 / 2672
-//   8.6 M of a 203x117x89 noise volume      - / 2042 / 1950
+// A wavefront launch costs some 0.25 ms more than its paths (0.5 ms with eight
+// bounces): four kernels a round and lane, most of them a few microseconds.
+// Here a round costs its block three barriers.  Per sample the block form is
+// the slower one: all four parts run at the registers of the largest (64, 1024
+// threads an SM), and a block of a thousand paths ends every DDA part waiting
+// for its longest segments.  Measured (us, thread per sample / block /
+// wavefront; the line to the wavefront is drawn in vt_api.cu, with more):
+//   19 k samples of 64^3 spheres          118 /  170 /    -
+//   262 k of 128^3 noise, 8 bounces       610 /  462 /  761
+//   1.05 M of 64^3 spheres                805 /  560 /  625
+//   2.1 M of a 203x117x89 noise volume   1477 /  694 /  896
+//   3.1 M of 128^3 noise                    - / 2248 / 1876
 // 512 slots against 1024: 545 and 568 us at 1.05 M samples, 748 and 676 at
 // 2.1 M: about a third of a block's samples in flight is best.
 // State fields of a path slot.
