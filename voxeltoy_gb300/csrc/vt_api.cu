@@ -126,6 +126,23 @@ uint64_t vt_context::trim(uint64_t keep) {
   return trim_locked(this, keep);
 }
 
+// The other lanes' streams and the events that fork and join them.
+int vt_context::ensure_lanes() {
+  if (lane_ready) return VT_OK;
+  cudaEvent_t ready = nullptr;
+  cudaError_t e = cudaEventCreateWithFlags(&ready, cudaEventDisableTiming);
+  for (int l = 0; l < kMaxLanes - 1 && e == cudaSuccess; ++l) {
+    if (!lane_stream[l]) e = cudaStreamCreateWithFlags(&lane_stream[l], cudaStreamNonBlocking);
+    if (e == cudaSuccess && !lane_done[l]) e = cudaEventCreateWithFlags(&lane_done[l], cudaEventDisableTiming);
+  }
+  if (e != cudaSuccess) {
+    if (ready) cudaEventDestroy(ready);
+    return cuda_fail(e, "lane streams");
+  }
+  lane_ready = ready;
+  return VT_OK;
+}
+
 int vt_context::ensure_scratch(size_t bytes) {
   if (scratch_bytes >= bytes) return VT_OK;
   release(scratch);
@@ -561,6 +578,11 @@ extern "C" int vt_scene_create_from_offsets(vt_context* ctx, int32_t rx, int32_t
   return rc;
 }
 
+// Voxels from which on a voxelization's fills get a stream of their own: the
+// 1.1 GB of a 1024^3 volume take 0.19 ms beside an upload of 23 MB, the events
+// some 5 us.
+constexpr int64_t kFillBeside = (int64_t)1 << 26;
+
 extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, int64_t n_vertices,
                                       const uint32_t* indices, int64_t n_triangles, int32_t rx, int32_t ry,
                                       int32_t rz, int32_t mode, int32_t placement, const vt_material* palette,
@@ -589,9 +611,18 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
   if (rc == VT_OK) rc = ctx->ensure_scratch(voxelize_scratch_bytes(n_triangles));
   if (rc == VT_OK) rc = ctx->alloc((void**)&s->bricks, sizeof(unsigned long long) * nb);
   if (rc != VT_OK) { ctx->release(d_v); ctx->release(d_i); delete s; return rc; }
-  cudaError_t e = cudaMemsetAsync(s->grid, 0, (size_t)nvox, ctx->stream);
+  // The fills of a large volume run beside the mesh's upload and preparation.
+  const bool beside = nvox >= kFillBeside && ctx->ensure_lanes() == VT_OK;
+  cudaStream_t fill = beside ? ctx->lane_stream[0] : ctx->stream;
+  cudaError_t e = cudaSuccess;
+  if (beside) {   // after whatever used the blocks before
+    e = cudaEventRecord(ctx->lane_ready, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(fill, ctx->lane_ready, 0);
+  }
+  if (e == cudaSuccess) e = cudaMemsetAsync(s->grid, 0, (size_t)nvox, fill);
   if (e == cudaSuccess)
-    e = launch_bricks_init(s->bricks, rx, ry, rz, s->bdim[0], s->bdim[1], s->bdim[2], scene_shape(s), ctx->stream);
+    e = launch_bricks_init(s->bricks, rx, ry, rz, s->bdim[0], s->bdim[1], s->bdim[2], scene_shape(s), fill);
+  if (e == cudaSuccess && beside) e = cudaEventRecord(ctx->lane_done[0], fill);
   if (e == cudaSuccess && n_vertices)
     e = cudaMemcpyAsync(d_v, vertices, sizeof(float) * 3 * n_vertices, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess && n_triangles)
@@ -600,6 +631,10 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
   if (e == cudaSuccess)
     e = launch_mesh_prep(d_v, n_vertices, d_i, n_triangles, placement == VT_MESH_FIT_UNIT_CUBE, rx, ry, rz, prep,
                          ctx->sm_count, ctx->stream);
+  if (beside) {   // also after an error: the fills end before the scene's blocks go back
+    const cudaError_t w = cudaStreamWaitEvent(ctx->stream, ctx->lane_done[0], 0);
+    if (e == cudaSuccess) e = w;
+  }
   if (e == cudaSuccess)
     e = launch_voxelize(d_v, n_vertices, d_i, n_triangles, rx, ry, rz, mode & 1,
                         (mode & VT_VOXELIZE_REFERENCE_BOUNDS) != 0, s->grid, 1, s->bricks, s->bdim[0], s->bdim[1],
@@ -1442,13 +1477,9 @@ static int wf_reserve(vt_context* ctx, int64_t slots, int64_t items) {
     int rc = ctx->alloc((void**)&ctx->wf_ctl, vt_context::kMaxLanes * kCtlBytes);
     if (rc != VT_OK) return rc;
   }
-  if (!ctx->lane_ready) {
-    cudaError_t e = cudaEventCreateWithFlags(&ctx->lane_ready, cudaEventDisableTiming);
-    for (int l = 0; l < vt_context::kMaxLanes - 1 && e == cudaSuccess; ++l) {
-      e = cudaStreamCreateWithFlags(&ctx->lane_stream[l], cudaStreamNonBlocking);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->lane_done[l], cudaEventDisableTiming);
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "lane streams");
+  {
+    int rc = ctx->ensure_lanes();
+    if (rc != VT_OK) return rc;
   }
   if (!ctx->h_live) {
     cudaError_t e = cudaHostAlloc((void**)&ctx->h_live, 64, cudaHostAllocDefault);

@@ -77,6 +77,7 @@ struct vt_context {
   uint64_t cached = 0;
   uint64_t cache_limit = 2ull << 30;
   int ensure_scratch(size_t bytes);
+  int ensure_lanes();
   int ensure_noise();
   void log(const char* fmt, ...);
 };
