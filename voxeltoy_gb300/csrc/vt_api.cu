@@ -1184,6 +1184,7 @@ int vt::build_frame(vt_job* j) {
     F.bmax[i] = s->bmax[i];
     F.vsize[i] = s->vsize[i];
     F.vext[i] = 1.0f / (s->bmax[i] - s->bmin[i]);
+    F.inv_res[i] = 1.0f / (float)s->res[i];
     F.bdim[i] = s->bdim[i];
     F.bsh[i] = s->bsh[i];
   }

@@ -122,12 +122,12 @@ VT_HD float reduce_pio2(float x, int* q) {
 VT_HD float vsin(float x) {
   int q; const float r = reduce_pio2(x, &q);
   const float s = sin_poly(r), c = cos_poly(r);
-  switch (q) { case 0: return s; case 1: return c; case 2: return -s; default: return -c; }
+  return u2f(f2u((q & 1) ? c : s) ^ ((uint32_t)(q & 2) << 30));          // s, c, -s, -c
 }
 VT_HD float vcos(float x) {
   int q; const float r = reduce_pio2(x, &q);
   const float s = sin_poly(r), c = cos_poly(r);
-  switch (q) { case 0: return c; case 1: return -s; case 2: return -c; default: return s; }
+  return u2f(f2u((q & 1) ? s : c) ^ ((uint32_t)((q + 1) & 2) << 30));    // c, -s, -c, s
 }
 
 // ---- log2 / exp2 / pow --------------------------------------------------------

@@ -54,6 +54,7 @@ struct Frame {
   float bmax[3];
   float vsize[3];            // (bmax-bmin)/res
   float vext[3];             // 1/(bmax-bmin), dda.h:16
+  float inv_res[3];          // 1/res
   int32_t bdim[3];           // brick grid dimensions
   int32_t bsh[3];            // log2 of a brick's extent along x, y, z (sum 6)
   float viewport[4];

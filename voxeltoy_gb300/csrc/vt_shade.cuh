@@ -25,6 +25,21 @@ constexpr float kPI = 3.14159265359f;
 constexpr float kTWO_PI = 6.28318530718f;
 constexpr float kINV_TWOPI = 0.15915494309f;
 
+// x / c for a divisor c known in advance, inv_c = 1 / c rounded to nearest:
+// the product with the reciprocal, corrected by its exact remainder
+// (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", 2004).  The
+// remainder is taken as q * c - x, so that a zero keeps its sign.  Three
+// operations against the nine or so of a general division.  Holds where the
+// remainder does not underflow and x is finite: for c = pi and 2 pi every
+// |x| > 4e-32 (all of them tried), for integers 0 <= x < c < 2^21 always (the
+// quotient is then at least 2^-22 of its last place from a rounding boundary,
+// the corrected product 1.5 * 2^-23 of it from the quotient).
+VT_D float div_known(float x, float c, float inv_c) {
+  const float q = x * inv_c;
+  return fmaf(-fmaf(q, c, -x), inv_c, q);
+}
+
 // ------------------------------------------------------------------ vectors
 struct v3 { float x, y, z; };
 VT_D v3 mk3(float x, float y, float z) { v3 r; r.x = x; r.y = y; r.z = z; return r; }
@@ -238,6 +253,21 @@ VT_D Basis voxel_basis(const Frame& F, int x, int y, int z, v3 ro, v3 rd, bool o
     mz = (!kx && !ky) ? 1.0f : 0.0f;
   }
   b.normal = mk3(mx * vtb::gsign(c2h.x), my * vtb::gsign(c2h.y), mz * vtb::gsign(c2h.z));
+  // The frame is binormal = normalize(cross(cross(n, (c, c, c)), n)) with c =
+  // 0.57735026919, tangent = normalize(cross(binormal, n)).  For a normal
+  // along one axis the cross products are the products of c and, after the
+  // first normalisation, of 0.70710677 with vectors of 0 and +-1, so the two
+  // normalisations are two constants: the same bits, the signs of zeros
+  // included, without six divisions and two roots.  With the known divisors
+  // (div_known) and the one division of the albedo: 1024^2 x 256 spp of 256^3
+  // noise 104.7 -> 98.8 ms, 512^2 x 1 spp 440 -> 417 us.
+  if (dot(b.normal, b.normal) == 1.0f) {
+    const v3 n = b.normal;
+    const v3 u = cross(mk3(n.y - n.z, n.z - n.x, n.x - n.y), n);
+    b.binormal = 0.70710677f * u;
+    b.tangent = 0.70710683f * cross(u, n);
+    return b;
+  }
   const float d3 = 0.57735026919f;
   const v3 tangent = cross(b.normal, mk3(d3, d3, d3));
   b.binormal = normalize(cross(tangent, b.normal));
@@ -586,7 +616,7 @@ VT_D float2 sample_disk(float u0, float u1) {
 VT_D float4 cosine_hemisphere(float u0, float u1) {
   const float2 p = sample_disk(u0, u1);
   const float y = sqrtf(vtb::gmax(0.0f, (1.0f - p.x * p.x) - p.y * p.y));
-  return make_float4(p.x, y, p.y, y / kPI);
+  return make_float4(p.x, y, p.y, div_known(y, kPI, 1.0f / kPI));   // y = 0 or > 1e-8
 }
 VT_D float4 uniform_hemisphere(float u0, float u1) {
   const float y = u0;
@@ -638,7 +668,7 @@ VT_D FPdf eval_bsdf(const Frame& F, const Mat& m, v3 wo, v3 wi) {
   FPdf r;
   if (m.type == 0) {                                                 // lambertian.h:23-29
     r.pdf = wi.y / kPI;
-    r.f = m.albedo / kPI;
+    r.f = m.albedo;                                                  // divided by pi already (ext_hit)
     return r;
   }
   if (m.type == 1 || m.type == 2) {                                  // microfacet.h:73-91
@@ -666,7 +696,7 @@ VT_D v3 sample_bsdf(const Frame& F, const JobDev& J, const Mat& m, v3 wo, Rng& r
   u_rr = u.z;
   if (m.type == 0) {                                                 // lambertian.h:10-19
     const float4 s = cosine_hemisphere(u.x, u.y);
-    out.f = m.albedo / kPI;
+    out.f = m.albedo;
     out.pdf = s.w;
     return mk3(s.x, s.y, s.z);
   }
@@ -698,9 +728,9 @@ VT_D v3 sample_bsdf(const Frame& F, const JobDev& J, const Mat& m, v3 wo, Rng& r
 VT_D float2 uv_from_dir(v3 v, float rot) {
   const float theta = vtb::vacos(v.y);
   const float phi = (vtb::vatan2(v.z, v.x) + kPI) + rot;
-  const float x = phi / kTWO_PI;
+  const float x = div_known(phi, kTWO_PI, 1.0f / kTWO_PI);   // below 4e-32 the lookup rounds it away
   const float u = x - 1.0f * floorf(x / 1.0f);
-  return make_float2(u, theta / kPI);
+  return make_float2(u, div_known(theta, kPI, 1.0f / kPI));   // theta = 0 or > 1e-5
 }
 VT_D v3 dir_from_uv(float u, float v, float rot) {
   const float phi = ((u * kTWO_PI) - kPI) - rot;
@@ -952,7 +982,8 @@ VT_D void light_sample(const Frame& F, const JobDev& J, Path& p, const Basis& b,
     const Mat lm = voxel_mat(F, J, ex, ey, ez, cnt);
     Ll = mk3(F.nee_scale, F.nee_scale, F.nee_scale) * lm.emission;
     const v3 res = mk3((float)F.res[0], (float)F.res[1], (float)F.res[2]);
-    v3 wp = (mk3((float)ex, (float)ey, (float)ez) / res) * (ld3(F.bmax) - ld3(F.bmin)) + ld3(F.bmin);
+    v3 wp = mk3(div_known((float)ex, res.x, F.inv_res[0]), div_known((float)ey, res.y, F.inv_res[1]),
+                div_known((float)ez, res.z, F.inv_res[2])) * (ld3(F.bmax) - ld3(F.bmin)) + ld3(F.bmin);
     wp = wp + mk3(u.y, u.z, u.w) * ld3(F.vsize);
     const v3 to_light = wp - b.position;
     const float r = length(to_light);
@@ -1060,7 +1091,8 @@ VT_D float wire_factor(const Frame& F, const Basis& b, int x, int y, int z) {
 template <bool kCount>
 VT_D void ext_hit(const Frame& F, const JobDev& J, Path& p, SegEnd e, Cnt<kCount>& cnt) {
   const Basis b = voxel_basis(F, e.x, e.y, e.z, p.ro, p.rd, !(F.quirks & Q_UNGUARDED));   // :220-223
-  const Mat m = voxel_mat(F, J, e.x, e.y, e.z, cnt);              // :225-226
+  Mat m = voxel_mat(F, J, e.x, e.y, e.z, cnt);                    // :225-226
+  if (m.type == 0) m.albedo = m.albedo / kPI;                     // lambertian.h:10-29, both of its uses
   const v3 wo = -p.rd;
   const v3 lwo = world_to_local(wo, b);
   if (p.bounces == 0) p.L = p.L + p.T * m.emission;               // :241-245
