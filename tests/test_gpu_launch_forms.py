@@ -89,3 +89,22 @@ def test_forms_agree_where_most_rays_miss(fctx, w, h):
     for i in range(3):
         cfg.camera.eye[i] = cfg.camera.eye[i] * 6.0
     compare(fctx, [cfg], 3)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (7, 3), (8, 4), (33, 65), (160, 121), (301, 203), (512, 300)])
+def test_edit_mode_images_are_their_samples(fctx, w, h):
+    """Edit-mode images, rendered in tiles of 8 x 1, 2 or 4 pixels by size,
+    against the samples that the pixel-per-thread diagnostic gives (compared
+    with the oracle elsewhere)."""
+    cfg = config2(w, h)
+    cfg.settings.wireframe_opacity = 0.6
+    scene, env, job = gpu_setup(fctx, cfg)
+    try:
+        job.set_integrator(1)
+        want = job.samples_diag(0)[0]
+        job.render(1)
+        assert np.array_equal(job.readback().view(np.uint32), want.view(np.uint32))
+        job.render(2)
+        assert job.samples() == 3
+    finally:
+        close_all(job, scene, env)
