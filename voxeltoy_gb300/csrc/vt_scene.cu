@@ -161,61 +161,80 @@ __global__ void k_cubes_large(uint32_t* __restrict__ e, int32_t words, int32_t p
   e[7 * n + i] = c16;
 }
 
-// One warp per word: lane 4 o + q gathers octant o of bricks 8 q .. 8 q + 7;
-// the bytes change places through shared memory into a word per brick.
-// A warp takes kCubeRun words in a row: its octants read eight rows of each
-// bitmap, and a sector holds eight words of one (a word per warp in turn
-// fetched every sector eight times: 200 us for 1024^3).
+// A warp takes four words at a time: lane 8 i + o reads octant o of word i,
+// eight bitmaps, and spreads the levels of its 32 bricks to a byte each, four
+// bricks a 32-bit word; through shared memory lane 8 i + g then gets those of
+// all octants for bricks 4 g .. 4 g + 3 of word i, and turns the 4 x 8 bytes
+// into a word per brick.  What bounds it is issue.  1024^3: 70 us; with a warp
+// per word, four lanes reading each octant and the bytes changing places one
+// by one, 158.  A warp takes kCubeRun words in a row, since a sector holds
+// eight words of a bitmap.
 constexpr int kCubeWarps = 4;
 constexpr uint32_t kCubeRun = 8;
+constexpr int kCubePitch = 72;   // 32-bit words between the four words' bytes: 64 and a shift of the banks
 __global__ void __launch_bounds__(32 * kCubeWarps) k_cubes_bytes(const uint32_t* __restrict__ e, int32_t words,
                                                                  int32_t px, int32_t py, int32_t pz,
                                                                  unsigned long long* __restrict__ runs) {
-  __shared__ __align__(8) uint8_t s[kCubeWarps][32][8];
+  __shared__ __align__(16) uint32_t s[kCubeWarps][4 * kCubePitch];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int o = lane >> 2, q = lane & 3;
+  const int o = lane & 7;
   const uint32_t n = (uint32_t)words * py * pz;
   const uint32_t first = (blockIdx.x * kCubeWarps + warp) * kCubeRun, last = min(n, first + kCubeRun);
+  if (first >= n) return;   // the whole warp
   const uint32_t down = ((o & 2) ? 0u : (uint32_t)words) + ((o & 4) ? 0u : (uint32_t)words * py);
-  const uint32_t row = first / (uint32_t)words;
-  int w = (int)(first - row * words), z = (int)(row / (uint32_t)py), y = (int)(row - (uint32_t)z * py);
-  for (uint32_t i = first; i < last; ++i) {
-    // the cube's lowest row lies (side - 1) rows and slices down where the
-    // octant's y, z point down: in the array if side - 1 is at most `low`
-    const int low = min((o & 2) ? kMaxFreeCube : y, (o & 4) ? kMaxFreeCube : z);
-    uint32_t c[kCubeSides];
+  uint32_t i = first + (lane >> 3);
+  const uint32_t row = i / (uint32_t)words;
+  int w = (int)(i - row * words), z = (int)(row / (uint32_t)py), y = (int)(row - (uint32_t)z * py);
+  uint32_t* const mine = &s[warp][(lane >> 3) * kCubePitch];
+  for (uint32_t i0 = first; i0 < last; i0 += 4, i += 4) {   // the same turns for every lane
+    if (i < last) {
+      // the cube's lowest row lies (side - 1) rows and slices down where the
+      // octant's y, z point down: in the array if side - 1 is at most `low`
+      const int low = min((o & 2) ? kMaxFreeCube : y, (o & 4) ? kMaxFreeCube : z);
+      uint32_t c[kCubeSides];
 #pragma unroll
-    for (int k = 0; k < kCubeSides; ++k) {   // every read is issued before any is used
-      const int off = kCubeSide[k] - 1;
-      const uint32_t* r = e + (size_t)k * n + (i - (uint32_t)off * down);
-      const bool in = off <= low;
-      const uint32_t cur = in ? r[0] : 0u, prev = in && !(o & 1) && w > 0 ? r[-1] : 0u;
-      c[k] = (o & 1) ? cur : __funnelshift_l(prev, cur, off);   // and from its lowest brick
-    }
-    // levels passed, 0 to 8, in four bit planes: each level implies the ones before it
-    const uint32_t b0 = (c[0] & ~c[1]) | (c[2] & ~c[3]) | (c[4] & ~c[5]) | (c[6] & ~c[7]);
-    const uint32_t b1 = (c[1] & ~c[3]) | (c[5] & ~c[7]);
-    const uint32_t b2 = c[3] & ~c[7], b3 = c[7];
-    uint32_t lo = 0u, hi = 0u;   // a byte per brick
+      for (int k = 0; k < kCubeSides; ++k) {   // every read is issued before any is used
+        const int off = kCubeSide[k] - 1;
+        const uint32_t* r = e + (size_t)k * n + (i - (uint32_t)off * down);
+        const bool in = off <= low;
+        const uint32_t cur = in ? r[0] : 0u, prev = in && !(o & 1) && w > 0 ? r[-1] : 0u;
+        c[k] = (o & 1) ? cur : __funnelshift_l(prev, cur, off);   // and from its lowest brick
+      }
+      // levels passed, 0 to 8, in four bit planes: each level implies the ones before it
+      const uint32_t b0 = (c[0] & ~c[1]) | (c[2] & ~c[3]) | (c[4] & ~c[5]) | (c[6] & ~c[7]);
+      const uint32_t b1 = (c[1] & ~c[3]) | (c[5] & ~c[7]);
+      const uint32_t b2 = c[3] & ~c[7], b3 = c[7];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t v = (k == 0 ? b0 : k == 1 ? b1 : k == 2 ? b2 : b3) >> (8 * q);
-      lo |= (((v & 15u) * 0x00204081u) & 0x01010101u) << k;
-      hi |= ((((v >> 4) & 15u) * 0x00204081u) & 0x01010101u) << k;
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      s[warp][8 * q + j][o] = (uint8_t)(lo >> (8 * j));
-      s[warp][8 * q + 4 + j][o] = (uint8_t)(hi >> (8 * j));
+      for (int g = 0; g < 8; ++g) {   // a byte per brick: bit j of a nibble to bit 8 j
+        uint32_t v = (((b0 >> (4 * g)) & 15u) * 0x00204081u) & 0x01010101u;
+        v |= (((b1 >> (4 * g)) & 15u) * 0x00408102u) & 0x02020202u;
+        v |= (((b2 >> (4 * g)) & 15u) * 0x00810204u) & 0x04040404u;
+        v |= (((b3 >> (4 * g)) & 15u) * 0x01020408u) & 0x08080808u;
+        mine[8 * g + o] = v;
+      }
     }
     __syncwarp();
-    const int x = 32 * w + lane;
-    if (x < px) runs[((int64_t)z * py + y) * px + x] = *(const unsigned long long*)s[warp][lane];
+    if (i < last) {
+      const int g = o;
+      const uint4 a = *(const uint4*)&mine[8 * g], b = *(const uint4*)&mine[8 * g + 4];
+      // bricks 0, 1 and (h) 2, 3 of octant pairs, then the pairs of each brick
+      const uint32_t a01 = __byte_perm(a.x, a.y, 0x5140), a23 = __byte_perm(a.z, a.w, 0x5140);
+      const uint32_t a01h = __byte_perm(a.x, a.y, 0x7362), a23h = __byte_perm(a.z, a.w, 0x7362);
+      const uint32_t b01 = __byte_perm(b.x, b.y, 0x5140), b23 = __byte_perm(b.z, b.w, 0x5140);
+      const uint32_t b01h = __byte_perm(b.x, b.y, 0x7362), b23h = __byte_perm(b.z, b.w, 0x7362);
+      const int x = 32 * w + 4 * g;
+      unsigned long long* at = runs + ((int64_t)z * py + y) * px + x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t pick = (j & 1) ? 0x7632u : 0x5410u;
+        const uint32_t lo = j < 2 ? __byte_perm(a01, a23, pick) : __byte_perm(a01h, a23h, pick);
+        const uint32_t hi = j < 2 ? __byte_perm(b01, b23, pick) : __byte_perm(b01h, b23h, pick);
+        if (x + j < px) at[j] = ((unsigned long long)hi << 32) | lo;
+      }
+    }
     __syncwarp();
-    if (++w == words) {
-      w = 0;
+    for (w += 4; w >= words; w -= words)
       if (++y == py) { y = 0; ++z; }
-    }
   }
 }
 
