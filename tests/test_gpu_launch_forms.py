@@ -108,3 +108,37 @@ def test_edit_mode_images_are_their_samples(fctx, w, h):
         assert job.samples() == 3
     finally:
         close_all(job, scene, env)
+
+
+def test_small_budgets_take_the_wavefront():
+    """A budget that holds the wavefront with few path slots, but not the block
+    form's state, still renders, and the same image; so does a wavefront launch
+    that needs the memory an earlier block launch kept."""
+    cfg = config2(400, 401)                    # block form: 160400 samples
+    big = config2(1200, 1000)                  # the wavefront by size
+    images = []
+    for budget in (0, 24 << 20):       # the block form wants 30 MB in all, the wavefront 9
+        with Context(0, hbm_budget_bytes=budget) as ctx:
+            ctx.set_tuning(path_slots=1024)
+            made = gpu_setup(ctx, cfg)
+            job = made[2]
+            try:
+                job.render(1)
+                images.append(job.readback())
+            finally:
+                close_all(made[2], made[0], made[1])
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+    images = []
+    for budget in (0, 204 << 20):      # 197 MB, and 22 that the block form keeps
+        with Context(0, hbm_budget_bytes=budget) as ctx:
+            a, b = gpu_setup(ctx, cfg), gpu_setup(ctx, big)
+            try:
+                a[2].render(1)
+                ctx.set_tuning(path_slots=300000)
+                b[2].render(2)
+                close_all(a[2], a[0], a[1])    # their memory is what the readback's buffer takes
+                a = (None, None, None)
+                images.append(b[2].readback())
+            finally:
+                close_all(a[2], a[0], a[1], b[2], b[0], b[1])
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))

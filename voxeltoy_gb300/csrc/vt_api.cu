@@ -1835,9 +1835,28 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
     if (items >= ((int64_t)1 << 32)) return fail(VT_EINVAL, "more than 2^32 samples in one launch");
     int64_t max_b = 0;
     for (const JobEntry& e : entries) max_b = std::max<int64_t>(max_b, e.F.max_bounces);
-    int rc = by_size && items <= kPathsItems ? paths_launch(ctx, entries, items)
-             : by_size && items * (max_b + 2) <= kBlockWork ? block_launch(ctx, entries, grids, items)
-                                             : wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
+    int rc = VT_OK;
+    bool wave = true;
+    if (by_size && items <= kPathsItems) {
+      rc = paths_launch(ctx, entries, items);
+      wave = false;
+    } else if (by_size && items * (max_b + 2) <= kBlockWork) {
+      rc = block_launch(ctx, entries, grids, items);
+      wave = rc == VT_EBUDGET || rc == VT_ENOMEM;
+      if (wave) cudaGetLastError();
+    }
+    // the wavefront also where the block form's state exceeds the budget or the
+    // device (with few path slots set it takes less), which it then has to itself
+    if (wave) {
+      rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
+      if ((rc == VT_EBUDGET || rc == VT_ENOMEM) && ctx->block_state) {
+        cudaGetLastError();
+        ctx->release(ctx->block_state);
+        ctx->block_state = nullptr;
+        ctx->block_bytes = 0;
+        rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
+      }
+    }
     if (rc != VT_OK) return rc;
   }
   return VT_OK;
