@@ -58,16 +58,17 @@ void vt_context::log(const char* fmt, ...) {
   log_fn(buf, log_user);
 }
 
-// Frees cached blocks, largest first, until at most `keep` bytes stay cached
+// Frees cached blocks, oldest first, until at most `keep` bytes stay cached
 // (the caller holds mu).
 static uint64_t trim_locked(vt_context* ctx, uint64_t keep) {
   uint64_t freed = 0;
   if (ctx->cached > keep) cudaSetDevice(ctx->device);
   while (ctx->cached > keep && !ctx->cache.empty()) {
-    auto it = std::prev(ctx->cache.end());
-    cudaFree(it->second);
+    auto it = ctx->by_age.begin()->second;
+    cudaFree(it->second.ptr);
     ctx->cached -= it->first;
     freed += it->first;
+    ctx->by_age.erase(ctx->by_age.begin());
     ctx->cache.erase(it);
   }
   return freed;
@@ -83,10 +84,11 @@ int vt_context::alloc(void** ptr, size_t bytes) {
                 (unsigned long long)in_use, (unsigned long long)bytes, (unsigned long long)budget);
   auto hit = cache.lower_bound(bytes);
   if (hit != cache.end() && hit->first <= bytes + bytes / 4 && (!budget || in_use + hit->first <= budget)) {
-    *ptr = hit->second;
+    *ptr = hit->second.ptr;
     sizes[*ptr] = hit->first;
     in_use += hit->first;
     cached -= hit->first;
+    by_age.erase(hit->second.released);
     cache.erase(hit);
     return VT_OK;
   }
@@ -116,7 +118,8 @@ void vt_context::release(void* ptr) {
   if (!caching || sz > cache_limit || !stream) { cudaFree(ptr); return; }
   // no kernel of this context still uses the block when another takes it
   if (cudaStreamSynchronize(stream) != cudaSuccess) { cudaGetLastError(); cudaFree(ptr); return; }
-  cache.emplace(sz, ptr);
+  by_age[releases] = cache.emplace(sz, CachedBlock{ptr, releases});
+  ++releases;
   cached += sz;
   trim_locked(this, cache_limit);
 }
