@@ -85,6 +85,22 @@ def test_leaps_change_no_pixel(fctx, res, kind):
         close_all(a, b)
 
 
+def test_leaps_where_the_cubes_are_built_in_long_runs(fctx):
+    """A volume of more than 2^18 bitmap words, whose cubes' slices are taken
+    eight at a time, with a last run that is not full."""
+    rng = np.random.default_rng(5)
+    vox = np.zeros((2059, 2061, 24), np.uint8)
+    vox[rng.integers(0, 2059, 3000), rng.integers(0, 2061, 3000), rng.integers(0, 24, 3000)] = 1
+    a, b = (Scene.dense(fctx, vox, PALETTE) for _ in range(2))
+    try:
+        b.set_brick_shape((1, 2, 3))
+        before = a.info().device_bytes
+        same(images(fctx, a, 61, 47, 2), images(fctx, b, 61, 47, 2))
+        assert a.info().device_bytes > before
+    finally:
+        close_all(a, b)
+
+
 @pytest.mark.parametrize("size", [(400, 401), (1024, 800)])
 def test_leaps_in_larger_launches(fctx, size):
     vox = volume("shell", (200, 180, 220))

@@ -93,7 +93,7 @@ size_t free_cube_scratch_bytes(int32_t bx, int32_t by, int32_t bz) {
 // Side 1, one warp per word: bit i set if brick 32 w + i of the row is empty.
 // (A bitmap has fewer than 2^31 words: 32-bit indices and divisions.)  Bound by
 // the read of the bricks, so a warp has four words' reads under way (one: 41 us
-// for 1024^3, SIDE1).
+// for 1024^3, four: 27).
 __global__ void __launch_bounds__(256) k_cubes_1(const unsigned long long* __restrict__ bricks, int32_t px, uint32_t n,
                                                  uint32_t words, uint32_t* __restrict__ e1) {
   const int lane = threadIdx.x & 31;
@@ -124,20 +124,21 @@ __device__ __forceinline__ unsigned long long cube_bits(const uint32_t* __restri
 
 // Sides 2, 3 and 4 from side 1, and behind the bitmaps the number of bricks
 // that start a cube of side 4 (in 32 parts); sides 6, 8, 12 and 16 from sides 3 and 4.
-// A thread takes a word of kCubeRunZ slices in turn: the bits of four rows of
+// A thread takes a word of kRun slices in turn: the bits of four rows of
 // a slice make its squares, the squares of up to four slices the cubes, so a
 // word costs four rows and not sixteen.  The counts go out once a warp.
-// 1024^3: 51 -> 14 us.
-constexpr int kCubeRunZ = 8;
+// 1024^3: 51 -> 14 us at eight slices; bitmaps of less than 2^18 words, which
+// would leave most of the chip idle then, take two (256^3: 11 us at eight, 5.7 at two).
+template <int kRun>
 __global__ void __launch_bounds__(128) k_cubes_small(uint32_t* __restrict__ e, int32_t words, int32_t py, int32_t pz) {
   const int64_t n = (int64_t)words * py * pz;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, slice = (uint32_t)words * py;
   const uint32_t run = i / slice, at = i - run * slice;   // the word of every slice of the run
   const int y = (int)(at / (uint32_t)words), w = (int)(at - (uint32_t)y * words);
-  const int z0 = (int)(run * kCubeRunZ);   // past the last slice: nothing to do
+  const int z0 = (int)(run * kRun);   // past the last slice: nothing to do
   uint32_t s2 = 0u, s3[2] = {0u, 0u}, s4[3] = {0u, 0u, 0u}, open = 0u;   // squares of the slices before, latest first
 #pragma unroll
-  for (int k = 0; k < kCubeRunZ + 3; ++k) {
+  for (int k = 0; k < kRun + 3; ++k) {
     uint32_t q2 = ~0u, q3 = ~0u, q4 = ~0u;
 #pragma unroll
     for (int dy = 0; dy < 4; ++dy) {
@@ -148,8 +149,8 @@ __global__ void __launch_bounds__(128) k_cubes_small(uint32_t* __restrict__ e, i
       q4 &= (uint32_t)(x2 & (x2 >> 2));
     }
     // cubes that end with this slice
-    if (k >= 1 && k <= kCubeRunZ && z0 + k - 1 < pz) e[n + (int64_t)(z0 + k - 1) * slice + at] = q2 & s2;
-    if (k >= 2 && k <= kCubeRunZ + 1 && z0 + k - 2 < pz)
+    if (k >= 1 && k <= kRun && z0 + k - 1 < pz) e[n + (int64_t)(z0 + k - 1) * slice + at] = q2 & s2;
+    if (k >= 2 && k <= kRun + 1 && z0 + k - 2 < pz)
       e[2 * n + (int64_t)(z0 + k - 2) * slice + at] = q3 & s3[0] & s3[1];
     if (k >= 3 && z0 + k - 3 < pz) {
       const uint32_t c4 = q4 & s4[0] & s4[1] & s4[2];
@@ -276,8 +277,10 @@ cudaError_t launch_free_cubes_open(const unsigned long long* bricks, int32_t bx,
   if (m != cudaSuccess) return m;
   k_cubes_1<<<(unsigned)std::min<int64_t>((n + 31) / 32, (int64_t)sm_count * 64), 256, 0, st>>>(bricks, bx + 2,
                                                                                              (uint32_t)n, words, e);
-  const int64_t runs = (int64_t)words * py * ((pz + kCubeRunZ - 1) / kCubeRunZ);
-  k_cubes_small<<<(unsigned)((runs + 127) / 128), 128, 0, st>>>(e, words, py, pz);
+  const int run = n < (1 << 18) ? 2 : 8;
+  const unsigned blocks = (unsigned)(((int64_t)words * py * ((pz + run - 1) / run) + 127) / 128);
+  if (run == 2) k_cubes_small<2><<<blocks, 128, 0, st>>>(e, words, py, pz);
+  else k_cubes_small<8><<<blocks, 128, 0, st>>>(e, words, py, pz);
   return cudaGetLastError();
 }
 
