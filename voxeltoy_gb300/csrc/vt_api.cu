@@ -607,13 +607,13 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
   // on the device, and the voxelizer sets the brick bits itself, so no
   // host pass over the mesh and no separate brick pass follow
   float* d_v = nullptr;
-  uint32_t* d_i = nullptr;
   const int64_t nb = (int64_t)(s->bdim[0] + 2) * (s->bdim[1] + 2) * (s->bdim[2] + 2);
-  rc = ctx->alloc((void**)&d_v, sizeof(float) * 3 * std::max<int64_t>(n_vertices, 1));
-  if (rc == VT_OK) rc = ctx->alloc((void**)&d_i, sizeof(uint32_t) * 3 * std::max<int64_t>(n_triangles, 1));
+  const size_t v_bytes = (sizeof(float) * 3 * (size_t)std::max<int64_t>(n_vertices, 1) + 255) / 256 * 256;
+  rc = ctx->alloc((void**)&d_v, v_bytes + sizeof(uint32_t) * 3 * (size_t)std::max<int64_t>(n_triangles, 1));
+  uint32_t* const d_i = (uint32_t*)((char*)d_v + v_bytes);
   if (rc == VT_OK) rc = ctx->ensure_scratch(voxelize_scratch_bytes(n_triangles));
   if (rc == VT_OK) rc = ctx->alloc((void**)&s->bricks, sizeof(unsigned long long) * nb);
-  if (rc != VT_OK) { ctx->release(d_v); ctx->release(d_i); delete s; return rc; }
+  if (rc != VT_OK) { ctx->release(d_v); delete s; return rc; }
   // The fills of a large volume run beside the mesh's upload and preparation.
   const bool beside = nvox >= kFillBeside && ctx->ensure_lanes() == VT_OK;
   cudaStream_t fill = beside ? ctx->lane_stream[0] : ctx->stream;
@@ -642,11 +642,9 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
     e = launch_voxelize(d_v, n_vertices, d_i, n_triangles, rx, ry, rz, mode & 1,
                         (mode & VT_VOXELIZE_REFERENCE_BOUNDS) != 0, s->grid, 1, s->bricks, s->bdim[0], s->bdim[1],
                         scene_shape(s), ctx->scratch, ctx->sm_count * 4, ctx->stream);
-  unsigned long long bad = 0ull;   // pageable destination: written when the copy returns
+  unsigned long long bad = 0ull;   // pageable destination: written, and the stream idle, when the copy returns
   if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, &prep->bad, sizeof(bad), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   ctx->release(d_v);
-  ctx->release(d_i);
   if (e != cudaSuccess) { delete s; return cuda_fail(e, "voxelization"); }
   if (bad) {
     delete s;
