@@ -1,0 +1,95 @@
+"""Scenes used by more than one stream: a server that renders a caller's scene
+while the caller's context is at work or edits it, jobs on one context that
+render another context's scene, and tables replaced behind a render."""
+import time
+
+import numpy as np
+import pytest
+
+from helpers import close_all
+from voxeltoy_gb300 import Context, Job, Scene, Server
+from voxeltoy_gb300 import _lib as L
+from voxeltoy_gb300 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+PALETTE = [S.lambert(0.95), S.lambert(0.0), S.lambert(0.5, emission=(6.0, 5.0, 4.0))]
+
+
+@pytest.fixture
+def sctx():
+    c = Context()
+    yield c
+    c.close()
+
+
+def room_job(ctx, room, w=64, h=64, rng_mode=L.VT_RNG_PHILOX):
+    """A job whose passes take milliseconds: up to 1024 bounces between the walls."""
+    s = S.physical_settings(1024, seed=5)
+    s.rng_mode = rng_mode
+    return Job(ctx, room, None, S.orbit_camera(distance=120.0), s, w, h)
+
+
+def make_room(ctx, edge=8):
+    vox = np.ones((edge,) * 3, np.uint8)
+    vox[1:-1, 1:-1, 1:-1] = 0
+    lights = [(edge - 1, y, x) for y in (2, 4) for x in (2, 5)]
+    for at in lights:
+        vox[at] = 3
+    emissive = np.array([x + edge * (y + edge * z) for z, y, x in lights], np.int32)
+    return Scene.dense(ctx, vox, PALETTE, emissive=emissive)
+
+
+def queue_work(ctx, job, seconds=1.0):
+    """About that much GPU time on the context's stream, queued without waiting."""
+    ctx.render_batch([job], 1, kernel=1)
+    job.synchronize()
+    t0 = time.perf_counter()
+    ctx.render_batch([job], 4, kernel=1)
+    job.synchronize()
+    passes = int(min(800, max(4, 4 * seconds / (time.perf_counter() - t0))))
+    ctx.render_batch([job], passes, kernel=1)
+
+
+def open_volume(edge=96):
+    """Nearly all of it free cubes, a little matter in the corners."""
+    vox = np.zeros((edge,) * 3, np.uint8)
+    vox[0, 0, 0] = vox[-1, -1, -1] = vox[0, -1, 0] = 1
+    return vox
+
+
+def image(ctx, scene, edge=64):
+    job = Job(ctx, scene, None, S.orbit_camera(distance=300.0), S.physical_settings(3, seed=2), edge, edge)
+    try:
+        job.render(2)
+        return job.readback()
+    finally:
+        job.close()
+
+
+def test_edit_beside_a_servers_first_render(sctx):
+    """A voxel set by the owner while a server renders the scene for the first
+    time is there in every later image."""
+    room = make_room(sctx)
+    busy = room_job(sctx, room)
+    vox = open_volume()
+    warm, scene = Scene.dense(sctx, vox, PALETTE), Scene.dense(sctx, vox, PALETTE)
+    srv = Server(sctx)
+    cam, settings = S.orbit_camera(distance=300.0), S.physical_settings(3)
+    try:
+        assert srv.wait(srv.submit(warm, None, cam, settings, 32, 32, 1), 60.0) == L.VT_OK
+        queue_work(sctx, busy)
+        ticket = srv.submit(scene, None, cam, settings, 32, 32, 1)
+        time.sleep(0.3)
+        scene.set_voxel(48, 48, 48, 1)
+        vox[48, 48, 48] = 1
+        assert srv.wait(ticket, 60.0) == L.VT_OK
+        ref = Scene.dense(sctx, vox, PALETTE)
+        ref.set_brick_shape((1, 2, 3))
+        try:
+            assert np.array_equal(image(sctx, scene).view(np.uint32), image(sctx, ref).view(np.uint32))
+        finally:
+            ref.close()
+    finally:
+        srv.close()
+        close_all(busy, room, warm, scene)

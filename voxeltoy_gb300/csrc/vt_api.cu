@@ -1365,11 +1365,8 @@ extern "C" int vt_job_set_integrator(vt_job* j, int32_t integrator) {
 // 9.3 ms; 256^3 noise (0.15) 1024^2 x 256 spp 123.4 -> 114.2 ms; 64^3 spheres
 // (0.08) 564 -> 575 us; 128^3 noise (0.006) 472 -> 497 us.
 constexpr double kOpenFraction = 0.1;
-static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
-  vt_scene* s = const_cast<vt_scene*>(scene);
-  std::lock_guard<std::mutex> g(s->runs_mu);
-  if (s->runs_tried || s->bsh[0] != 2 || s->bsh[1] != 2 || s->bsh[2] != 2) return VT_OK;
-  s->runs_tried = true;
+static int build_free_cubes(vt_context* ctx, vt_scene* s) {
+  if (s->bsh[0] != 2 || s->bsh[1] != 2 || s->bsh[2] != 2) return VT_OK;
   if (s->ctx->budget || !s->ctx->free_cubes) return VT_OK;
   const int32_t bx = s->bdim[0], by = s->bdim[1], bz = s->bdim[2];
   void* scratch = nullptr;
@@ -1398,6 +1395,17 @@ static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
   s->runs.store((unsigned long long*)runs);
   s->generation += 1;   // jobs rebuild their frames before their next pass
   return VT_OK;
+}
+
+static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
+  vt_scene* s = const_cast<vt_scene*>(scene);
+  // without the lock, which an edit holds until its stream is idle
+  if (s->runs_tried) return VT_OK;
+  std::lock_guard<std::mutex> g(s->runs_mu);
+  if (s->runs_tried) return VT_OK;
+  const int rc = build_free_cubes(ctx, s);
+  s->runs_tried = true;
+  return rc;
 }
 
 // DDA steps between refills of a launch: the caller's choice, or 16, 8 where a
@@ -1968,6 +1976,9 @@ extern "C" int vt_scene_set_voxel(vt_scene* s, int32_t x, int32_t y, int32_t z, 
   VT_CHECK_ARG(entry >= 0 && entry <= s->n_palette, "entry outside the palette");
   vt_context* ctx = s->ctx;
   cudaSetDevice(ctx->device);
+  // held until the edit is done: free cubes that another stream builds (a
+  // server's first render of the scene) see it, or are there to be lowered
+  std::lock_guard<std::mutex> g(s->runs_mu);
   const int64_t idx = (int64_t)x + (int64_t)s->res[0] * ((int64_t)y + (int64_t)s->res[1] * z);
   VT_CUDA(launch_set_voxel(s->grid, s->bricks, s->res[0], s->res[1], s->bdim[0], s->bdim[1], scene_shape(s), x, y,
                            z, (uint8_t)entry, ctx->stream), "voxel edit");
@@ -1985,8 +1996,8 @@ extern "C" int vt_scene_set_voxel(vt_scene* s, int32_t x, int32_t y, int32_t z, 
     list.erase(std::remove(list.begin(), list.end(), (int32_t)idx), list.end());
     if ((int64_t)list.size() != s->n_emissive) rc = scene_emissive(ctx, s, list.data(), (int64_t)list.size(), 0);
   }
-  if (rc != VT_OK) return rc;
   VT_CUDA(cudaStreamSynchronize(ctx->stream), "voxel edit");
+  if (rc != VT_OK) return rc;
   s->generation += 1;
   return VT_OK;
 }
@@ -2225,6 +2236,7 @@ extern "C" int vt_scene_set_brick_shape(vt_scene* s, int32_t sx, int32_t sy, int
   if (sx == s->bsh[0] && sy == s->bsh[1] && sz == s->bsh[2]) return VT_OK;
   vt_context* ctx = s->ctx;
   cudaSetDevice(ctx->device);
+  std::lock_guard<std::mutex> g(s->runs_mu);   // no free cubes are built from the bricks meanwhile
   const int32_t old[3] = {s->bsh[0], s->bsh[1], s->bsh[2]};
   s->bsh[0] = sx; s->bsh[1] = sy; s->bsh[2] = sz;
   int32_t bdim[3];
@@ -2244,13 +2256,11 @@ extern "C" int vt_scene_set_brick_shape(vt_scene* s, int32_t sx, int32_t sy, int
   const int64_t old_nb = (int64_t)(s->bdim[0] + 2) * (s->bdim[1] + 2) * (s->bdim[2] + 2);
   ctx->release(s->bricks);
   s->bricks = bricks;
-  {   // the free cubes are those of the old shape
-    std::lock_guard<std::mutex> g(s->runs_mu);
-    unsigned long long* runs = s->runs.exchange(nullptr);
-    if (runs) s->bytes -= sizeof(unsigned long long) * (uint64_t)old_nb;
-    ctx->release(runs);
-    s->runs_tried = false;
-  }
+  // the free cubes are those of the old shape
+  unsigned long long* runs = s->runs.exchange(nullptr);
+  if (runs) s->bytes -= sizeof(unsigned long long) * (uint64_t)old_nb;
+  ctx->release(runs);
+  s->runs_tried = false;
   for (int i = 0; i < 3; ++i) s->bdim[i] = bdim[i];
   s->bytes = s->bytes - sizeof(unsigned long long) * (uint64_t)old_nb + sizeof(unsigned long long) * (uint64_t)nb;
   s->generation++;   // jobs on this scene rebuild their frames before their next pass

@@ -105,8 +105,8 @@ struct vt_scene {
   std::atomic<uint64_t> generation{0};   // bumped by edits that move device buffers
   // free cubes (vt_internal.h), built by the first render of the scene
   std::atomic<unsigned long long*> runs{nullptr};
-  bool runs_tried = false;       // built, or not to be had (under runs_mu)
-  std::mutex runs_mu;
+  std::atomic<bool> runs_tried{false};   // built, or not to be had
+  std::mutex runs_mu;            // held while they are built and while the bricks change
   std::vector<vt_material> host_palette;
   // the reference's flat material table and the record offset of each
   // palette entry in it (-1: the entry has no record there)
