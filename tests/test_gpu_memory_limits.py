@@ -1,0 +1,53 @@
+"""Renders and builds where device memory is short: on the device, and under a
+context's budget."""
+import numpy as np
+import pytest
+
+from helpers import close_all, gpu_setup, small_config2
+from voxeltoy_gb300 import Context, Job, Scene
+from voxeltoy_gb300 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+PALETTE = [S.lambert(0.7)]
+
+
+def open_volume(edge):
+    vox = np.zeros((edge,) * 3, np.uint8)
+    vox[0, 0, 0] = vox[-1, -1, -1] = vox[edge // 2, edge // 2, edge // 2] = 1
+    return vox
+
+
+@pytest.mark.parametrize("integrator", [0, 1])
+def test_a_render_goes_on_where_free_cubes_find_no_memory(integrator):
+    """The first render of an open scene on a device without room for its free
+    cubes succeeds without them, and counts its samples."""
+    torch = pytest.importorskip("torch")
+    vox = open_volume(512)
+    cam, s = S.orbit_camera(distance=500.0), S.physical_settings(3, seed=4)
+    with Context() as ctx:
+        a, b = (Scene.dense(ctx, vox, PALETTE) for _ in range(2))
+        jobs = [Job(ctx, sc, None, cam, s, 64, 48) for sc in (a, b)]
+        held = []
+        try:
+            before = b.info().device_bytes
+            for j in jobs:
+                j.set_integrator(integrator)
+            jobs[0].render(1)                      # its kernels are loaded, its buffers there
+            want = jobs[0].readback()
+            jobs[1].readback()
+            assert a.info().device_bytes > before
+            ctx.trim()
+            size = torch.cuda.mem_get_info()[0]
+            while size >= 1 << 21:                 # the rest of the device, down to 2 MB
+                try:
+                    held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+                except torch.cuda.OutOfMemoryError:
+                    size //= 2
+            jobs[1].render(1)
+            assert jobs[1].samples() == 1 and b.info().device_bytes == before
+            assert np.array_equal(jobs[1].readback().view(np.uint32), want.view(np.uint32))
+        finally:
+            held.clear()
+            torch.cuda.empty_cache()
+            close_all(*jobs, a, b)

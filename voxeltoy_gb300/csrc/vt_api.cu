@@ -36,7 +36,11 @@ int vt::fail(int code, const char* fmt, ...) {
   return code;
 }
 
+// Reports a failed CUDA call, which is then no longer the runtime's last error:
+// a caller that goes on without what failed (free cubes, lanes, the block form)
+// does not find it at its next launch.
 int vt::cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();
   return fail(e == cudaErrorMemoryAllocation ? VT_ENOMEM : VT_EDEVICE, "%s: %s", what, cudaGetErrorString(e));
 }
 
@@ -1852,14 +1856,12 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
     } else if (by_size && items * (max_b + 2) <= kBlockWork) {
       rc = block_launch(ctx, entries, grids, items);
       wave = rc == VT_EBUDGET || rc == VT_ENOMEM;
-      if (wave) cudaGetLastError();
     }
     // the wavefront also where the block form's state exceeds the budget or the
     // device (with few path slots set it takes less), which it then has to itself
     if (wave) {
       rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
       if ((rc == VT_EBUDGET || rc == VT_ENOMEM) && ctx->block_state) {
-        cudaGetLastError();
         ctx->release(ctx->block_state);
         ctx->block_state = nullptr;
         ctx->block_bytes = 0;
