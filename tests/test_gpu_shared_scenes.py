@@ -93,3 +93,28 @@ def test_edit_beside_a_servers_first_render(sctx):
     finally:
         srv.close()
         close_all(busy, room, warm, scene)
+
+
+def test_edit_after_a_render_on_another_context(sctx):
+    """A job on one context renders another context's scene; an edit of the
+    scene after the call is not in its image."""
+    room = make_room(sctx)
+    with Context() as other:
+        job = room_job(other, room)
+        try:
+            job.render(1)
+            job.synchronize()
+            want = job.readback()
+            job.reset()
+            job.synchronize()
+            job.render(1)
+            for y in range(1, 7):
+                for z in range(1, 7):
+                    room.set_voxel(0, y, z, 2)            # a white wall turns black
+            assert np.array_equal(job.readback().view(np.uint32), want.view(np.uint32))
+            job.reset()
+            job.render(1)
+            assert not np.array_equal(job.readback().view(np.uint32), want.view(np.uint32))
+        finally:
+            job.close()
+    room.close()

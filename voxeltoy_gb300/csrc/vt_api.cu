@@ -1819,6 +1819,12 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
     return VT_OK;
   }
   std::vector<int32_t> done(n, 0);
+  // the owner of another context's scene or environment cannot order its edits
+  // and releases after this stream: as the other forms do, a launch without
+  // rounds then ends with the last read of them
+  bool foreign = false;
+  for (int i = 0; i < n; ++i)
+    foreign = foreign || jobs[i]->scene->ctx != ctx || (jobs[i]->env && jobs[i]->env->ctx != ctx);
   const int64_t slots_cap = slots > 0 ? slots : ctx->max_slots;
   for (;;) {
     int64_t pix_left = 0;
@@ -1852,6 +1858,7 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
     bool wave = true;
     if (by_size && items <= kPathsItems) {
       rc = paths_launch(ctx, entries, items);
+      if (rc == VT_OK && foreign) VT_CUDA(cudaStreamSynchronize(ctx->stream), "samples");
       wave = false;
     } else if (by_size && items * (max_b + 2) <= kBlockWork) {
       rc = block_launch(ctx, entries, grids, items);
