@@ -118,3 +118,28 @@ def test_edit_after_a_render_on_another_context(sctx):
         finally:
             job.close()
     room.close()
+
+
+def test_noise_table_replaced_after_a_render(sctx):
+    """A render uses the noise table of its call."""
+    room = make_room(sctx)
+    job = room_job(sctx, room, rng_mode=L.VT_RNG_NOISE_TABLE)
+    table = sctx.noise_table()
+    other = np.ascontiguousarray(table[::-1, ::-1])
+    put = lambda t: L.call("vt_diag_set_noise_table", sctx.h, L.ptr(t), t.nbytes)
+    try:
+        job.render(1)
+        want = job.readback()
+        for _ in range(4):
+            job.reset()
+            job.synchronize()
+            job.render(1)
+            put(other)
+            assert np.array_equal(job.readback().view(np.uint32), want.view(np.uint32))
+            put(table)
+        put(other)
+        job.reset()
+        job.render(1)
+        assert not np.array_equal(job.readback().view(np.uint32), want.view(np.uint32))
+    finally:
+        close_all(job, room)

@@ -2415,6 +2415,7 @@ extern "C" int vt_diag_set_noise_table(vt_context* ctx, const float* rgba, size_
   VT_CHECK_ARG(bytes >= n, "table must hold 1024*1024 RGBA floats");
   int rc = ctx->ensure_noise();
   if (rc != VT_OK) return rc;
+  VT_CUDA(cudaStreamSynchronize(ctx->stream), "noise table");   // launches under way keep the old one
   VT_CUDA(cudaMemcpy(ctx->noise, rgba, n, cudaMemcpyHostToDevice), "noise table");
   return VT_OK;
 }
