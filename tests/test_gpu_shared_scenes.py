@@ -95,6 +95,57 @@ def test_edit_beside_a_servers_first_render(sctx):
         close_all(busy, room, warm, scene)
 
 
+def test_servers_first_render_leaves_the_owners_stream_alone(sctx):
+    """A server's first render of a scene finishes while its owner's stream is
+    still at work."""
+    room = make_room(sctx)
+    busy = room_job(sctx, room)
+    warm, scene = (Scene.dense(sctx, open_volume(), PALETTE) for _ in range(2))
+    srv = Server(sctx)
+    cam, settings = S.orbit_camera(distance=300.0), S.physical_settings(3)
+    try:
+        assert srv.wait(srv.submit(warm, None, cam, settings, 32, 32, 1), 60.0) == L.VT_OK
+        before = scene.info().device_bytes
+        queue_work(sctx, busy, 2.0)
+        ticket = srv.submit(scene, None, cam, settings, 32, 32, 1)
+        assert srv.wait(ticket, 60.0) == L.VT_OK
+        t0 = time.perf_counter()
+        busy.synchronize()
+        assert time.perf_counter() - t0 > 0.3
+        assert scene.info().device_bytes > before         # with free cubes
+    finally:
+        srv.close()
+        close_all(busy, room, warm, scene)
+
+
+def test_owner_renders_beside_servers_first_renders(sctx):
+    """Launches that the owner replays as a graph go on, and give the same
+    image, while a server renders the owner's scenes for the first time."""
+    room = make_room(sctx, 24)
+    s = S.physical_settings(8, seed=5)
+    job = Job(sctx, room, None, S.orbit_camera(distance=120.0), s, 64, 64)
+    scenes = [Scene.dense(sctx, open_volume(64), PALETTE) for _ in range(40)]
+    srv = Server(sctx)
+    cam, settings = S.orbit_camera(distance=300.0), S.physical_settings(3)
+
+    def frame():
+        job.reset()
+        sctx.render_batch([job], 8, kernel=2, path_slots=1024)
+        return job.readback().view(np.uint32)
+    try:
+        want = frame()
+        for scene in scenes:
+            ticket = srv.submit(scene, None, cam, settings, 16, 16, 1)
+            while True:
+                assert np.array_equal(frame(), want)
+                if srv.poll(ticket)[0] not in (0, 1):     # queued, running
+                    break
+            assert srv.wait(ticket, 60.0) == L.VT_OK
+    finally:
+        srv.close()
+        close_all(job, room, *scenes)
+
+
 def test_edit_after_a_render_on_another_context(sctx):
     """A job on one context renders another context's scene; an edit of the
     scene after the call is not in its image."""

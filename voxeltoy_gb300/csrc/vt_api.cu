@@ -110,7 +110,7 @@ int vt_context::alloc(void** ptr, size_t bytes) {
   return VT_OK;
 }
 
-void vt_context::release(void* ptr) {
+void vt_context::release(void* ptr, bool idle) {
   if (!ptr) return;
   std::lock_guard<std::mutex> g(mu);
   auto it = sizes.find(ptr);
@@ -121,7 +121,7 @@ void vt_context::release(void* ptr) {
   cudaSetDevice(device);
   if (!caching || sz > cache_limit || !stream) { cudaFree(ptr); return; }
   // no kernel of this context still uses the block when another takes it
-  if (cudaStreamSynchronize(stream) != cudaSuccess) { cudaGetLastError(); cudaFree(ptr); return; }
+  if (!idle && cudaStreamSynchronize(stream) != cudaSuccess) { cudaGetLastError(); cudaFree(ptr); return; }
   by_age[releases] = cache.emplace(sz, CachedBlock{ptr, releases});
   ++releases;
   cached += sz;
@@ -1360,7 +1360,10 @@ extern "C" int vt_job_set_integrator(vt_job* j, int32_t integrator) {
 }
 
 // The free cubes of a scene about to be rendered, built on the rendering
-// context's stream and kept with the scene.  They only speed the DDA up: none
+// context's stream and kept with the scene, in memory of the scene's context.
+// The thread may be a server's, with the scene's context at work on another:
+// that one's allocator is taken, which is locked, but nothing waits for its
+// stream (which may be capturing).  They only speed the DDA up: none
 // for other brick shapes, for scenes of a context with a memory budget (the
 // budget is the caller's to spend), where memory is short, or where too little
 // of the volume is open for a leap to pay: the line lies at a tenth of the
@@ -1374,7 +1377,7 @@ static int build_free_cubes(vt_context* ctx, vt_scene* s) {
   if (s->ctx->budget || !s->ctx->free_cubes) return VT_OK;
   const int32_t bx = s->bdim[0], by = s->bdim[1], bz = s->bdim[2];
   void* scratch = nullptr;
-  if (s->ctx->alloc(&scratch, free_cube_scratch_bytes(bx, by, bz)) != VT_OK) return VT_OK;
+  if (ctx->alloc(&scratch, free_cube_scratch_bytes(bx, by, bz)) != VT_OK) return VT_OK;
   uint32_t* d_open = nullptr;
   uint32_t open[32];   // pageable: the read has completed when the copy returns
   cudaError_t e = launch_free_cubes_open(s->bricks, bx, by, bz, scratch, &d_open, ctx->sm_count, ctx->stream);
@@ -1386,12 +1389,12 @@ static int build_free_cubes(vt_context* ctx, vt_scene* s) {
   void* runs = nullptr;
   if (e == cudaSuccess && n_open >= kOpenFraction * bx * by * bz && s->ctx->alloc(&runs, bytes) == VT_OK) {
     e = launch_free_cubes(bx, by, bz, scratch, (unsigned long long*)runs, ctx->stream);
-    // other streams may render the scene next, and the scratch goes back
+    // other streams may render the scene next
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   }
-  s->ctx->release(scratch);
+  ctx->release(scratch);
   if (e != cudaSuccess) {
-    s->ctx->release(runs);
+    s->ctx->release(runs, /*idle=*/true);   // its only user is ctx's stream, which the line above waited for
     return cuda_fail(e, "free cubes");
   }
   if (!runs) return VT_OK;
