@@ -629,7 +629,8 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
   if (e == cudaSuccess) e = cudaMemsetAsync(s->grid, 0, (size_t)nvox, fill);
   if (e == cudaSuccess)
     e = launch_bricks_init(s->bricks, rx, ry, rz, s->bdim[0], s->bdim[1], s->bdim[2], scene_shape(s), fill);
-  if (e == cudaSuccess && beside) e = cudaEventRecord(ctx->lane_done[0], fill);
+  // recorded also after an error, which may have followed queued work
+  const cudaError_t filled = beside ? cudaEventRecord(ctx->lane_done[0], fill) : cudaSuccess;
   if (e == cudaSuccess && n_vertices)
     e = cudaMemcpyAsync(d_v, vertices, sizeof(float) * 3 * n_vertices, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess && n_triangles)
@@ -639,7 +640,8 @@ extern "C" int vt_scene_voxelize_mesh(vt_context* ctx, const float* vertices, in
     e = launch_mesh_prep(d_v, n_vertices, d_i, n_triangles, placement == VT_MESH_FIT_UNIT_CUBE, rx, ry, rz, prep,
                          ctx->sm_count, ctx->stream);
   if (beside) {   // also after an error: the fills end before the scene's blocks go back
-    const cudaError_t w = cudaStreamWaitEvent(ctx->stream, ctx->lane_done[0], 0);
+    const cudaError_t w = filled == cudaSuccess ? cudaStreamWaitEvent(ctx->stream, ctx->lane_done[0], 0) : filled;
+    if (w != cudaSuccess) cudaStreamSynchronize(fill);
     if (e == cudaSuccess) e = w;
   }
   if (e == cudaSuccess)
