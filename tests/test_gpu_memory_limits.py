@@ -51,3 +51,31 @@ def test_a_render_goes_on_where_free_cubes_find_no_memory(integrator):
             held.clear()
             torch.cuda.empty_cache()
             close_all(*jobs, a, b)
+
+
+def test_block_wavefront_state_gives_way_under_a_budget():
+    """What a launch as block wavefronts keeps for the next one counts against
+    the budget, and is given up for a scene, a job or a readback that needs it;
+    the next launch then is the wavefront, with the few path slots that fit."""
+    cfg = small_config2(edge=24, w=400, h=401, seed=11)
+    vox = open_volume(200)
+    used = 0
+    for budget in (0, 1):
+        with Context(0, hbm_budget_bytes=budget and used) as ctx:
+            ctx.set_tuning(path_slots=1024)
+            scene, env, job = gpu_setup(ctx, cfg)
+            more = []
+            try:
+                job.render(1)
+                used = ctx.memory() + (1 << 20)    # a MB beside what the render keeps
+                if budget:
+                    image = job.readback()         # a buffer of 2.6 MB
+                    more.append(Scene.dense(ctx, vox, PALETTE))                            # 8 MB
+                    more.append(Job(ctx, more[0], None, cfg.camera, cfg.settings, 400, 400))   # 5 MB
+                    job.render(1)
+                    assert job.samples() == 2
+                else:
+                    want = job.readback()
+            finally:
+                close_all(*more[::-1], job, scene, env)
+    assert np.array_equal(image.view(np.uint32), want.view(np.uint32))

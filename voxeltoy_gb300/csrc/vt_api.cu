@@ -79,6 +79,17 @@ static uint64_t trim_locked(vt_context* ctx, uint64_t keep) {
 }
 
 int vt_context::alloc(void** ptr, size_t bytes) {
+  int rc = take(ptr, bytes);
+  if ((rc == VT_EBUDGET || rc == VT_ENOMEM) && block_state) {   // idle: a block launch waits for its kernel
+    release(block_state);
+    block_state = nullptr;
+    block_bytes = 0;
+    rc = take(ptr, bytes);
+  }
+  return rc;
+}
+
+int vt_context::take(void** ptr, size_t bytes) {
   *ptr = nullptr;
   if (bytes == 0) bytes = 16;
   bytes = (bytes + 511) / 512 * 512;
@@ -1389,7 +1400,7 @@ static int build_free_cubes(vt_context* ctx, vt_scene* s) {
   for (uint32_t v : open) n_open += v;
   const size_t bytes = sizeof(unsigned long long) * (size_t)(bx + 2) * (by + 2) * (bz + 2);
   void* runs = nullptr;
-  if (e == cudaSuccess && n_open >= kOpenFraction * bx * by * bz && s->ctx->alloc(&runs, bytes) == VT_OK) {
+  if (e == cudaSuccess && n_open >= kOpenFraction * bx * by * bz && s->ctx->take(&runs, bytes) == VT_OK) {
     e = launch_free_cubes(bx, by, bz, scratch, (unsigned long long*)runs, ctx->stream);
     // other streams may render the scene next
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1870,16 +1881,8 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
       wave = rc == VT_EBUDGET || rc == VT_ENOMEM;
     }
     // the wavefront also where the block form's state exceeds the budget or the
-    // device (with few path slots set it takes less), which it then has to itself
-    if (wave) {
-      rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
-      if ((rc == VT_EBUDGET || rc == VT_ENOMEM) && ctx->block_state) {
-        ctx->release(ctx->block_state);
-        ctx->block_state = nullptr;
-        ctx->block_bytes = 0;
-        rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
-      }
-    }
+    // device (with few path slots set it takes less)
+    if (wave) rc = wf_launch(ctx, entries, grids, items, slots_cap, blocks_per_sm, count);
     if (rc != VT_OK) return rc;
   }
   return VT_OK;

@@ -70,10 +70,13 @@ struct vt_context {
   // longer asked for gave the grid of every 1024^3 volume back to the device
   // and took it again, 0.8 ms a volume); alloc takes the smallest cached block of
   // the rounded size up to a quarter larger before it calls cudaMalloc, and
-  // live plus cached bytes stay within the budget.  Both are safe from any
-  // thread; one that is not the context's own passes idle = true, for a block
-  // that nothing uses any more, and no stream is waited for.
+  // live plus cached bytes stay within the budget.  A request that finds no
+  // room gets the block wavefront's state, which is kept between launches only
+  // to be at hand.  From a thread that is not the context's own: take, which
+  // leaves that state alone, and release with idle = true, which waits for no
+  // stream, for a block that nothing uses any more.
   int alloc(void** ptr, size_t bytes);
+  int take(void** ptr, size_t bytes);
   void release(void* ptr, bool idle = false);
   uint64_t trim(uint64_t keep);           // free cached blocks down to `keep` bytes; returns bytes freed
   bool free_cubes = true;       // scenes of this context may hold free cubes
