@@ -241,7 +241,7 @@ typedef struct vt_scene_info {
   float voxel_size[3];
   int64_t n_emissive;     /* after pruning */
   int32_t n_palette;
-  uint64_t device_bytes;
+  uint64_t device_bytes;       /* held on the device; see vt_job_render         */
 } vt_scene_info;
 VT_API int vt_scene_get_info(const vt_scene* scene, vt_scene_info* info);
 /* Copy the byte-per-voxel grid back to the host (rx*ry*rz bytes). */
@@ -436,7 +436,16 @@ VT_API int vt_job_set_integrator(vt_job* job, int32_t integrator);
 /* Renderer::render (renderer.cpp:556-645) called `passes` times: each pass
  * adds one sample per pixel until max_samples are accumulated.  *result
  * receives VT_SAMPLES_PENDING or VT_FINISHED_RENDERING.  The call queues GPU
- * work and returns; vt_job_synchronize or a readback waits for it. */
+ * work and returns; vt_job_synchronize or a readback waits for it.
+ *
+ * The first render of a scene, by this or any other call that renders (a
+ * server's too), looks for empty cubes of its 4x4x4 bricks that rays can
+ * cross in one step.  A scene open enough for them to pay keeps them in eight
+ * bytes a brick (137 MB for 1024^3), counted in its device_bytes and in
+ * vt_context_memory from then on; the search itself takes up to one byte a
+ * brick of working memory, returned at once.  There are none for scenes of a
+ * context with a budget, for volumes that a server with a budget keeps, and
+ * where the memory is not to be had; images are the same without. */
 VT_API int vt_job_render(vt_job* job, int32_t passes, int32_t* result);
 VT_API int vt_job_synchronize(vt_job* job);
 VT_API int vt_job_sample_count(const vt_job* job, int32_t* samples);

@@ -79,3 +79,22 @@ def test_block_wavefront_state_gives_way_under_a_budget():
             finally:
                 close_all(*more[::-1], job, scene, env)
     assert np.array_equal(image.view(np.uint32), want.view(np.uint32))
+
+
+def test_device_bytes_count_the_free_cubes():
+    """The first render of an open scene adds eight bytes a padded brick."""
+    with Context() as ctx:
+        scene = Scene.dense(ctx, open_volume(96), PALETTE)
+        job = Job(ctx, scene, None, S.orbit_camera(), S.physical_settings(2), 32, 32)
+        try:
+            before, held = scene.info().device_bytes, ctx.memory()
+            for _ in range(2):
+                job.render(1)
+                assert scene.info().device_bytes == before + 8 * 26 ** 3
+            assert ctx.memory() - held >= 8 * 26 ** 3
+            scene.set_brick_shape((1, 2, 3))
+            job.render(1)
+            scene.set_brick_shape((2, 2, 2))
+            assert scene.info().device_bytes == before
+        finally:
+            close_all(job, scene)

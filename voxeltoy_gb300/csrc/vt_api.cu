@@ -282,6 +282,7 @@ extern "C" int vt_set_log_callback(vt_context* ctx, vt_log_fn fn, void* user) {
 
 extern "C" int vt_context_memory(const vt_context* ctx, uint64_t* bytes) {
   VT_CHECK_ARG(ctx && bytes, "null argument");
+  std::lock_guard<std::mutex> g(ctx->mu);
   *bytes = ctx->in_use;
   return VT_OK;
 }

@@ -23,7 +23,7 @@ struct vt_context {
   int kernel = 0;               // 0 by the launch's size, 1 plain, 2 wavefront
   vt_log_fn log_fn = nullptr;
   void* log_user = nullptr;
-  std::mutex mu;
+  mutable std::mutex mu;
   std::unordered_map<void*, size_t> sizes;
   float4* noise = nullptr;
   void* scratch = nullptr;      // reusable device scratch for diagnostics and picks
@@ -105,7 +105,7 @@ struct vt_scene {
   int32_t n_palette = 0;
   int32_t* emissive = nullptr;
   int64_t n_emissive = 0;
-  uint64_t bytes = 0;
+  std::atomic<uint64_t> bytes{0};        // a server's thread may add the free cubes'
   uint32_t flags = 0;            // creation flags (emissive list policy for edits)
   std::atomic<uint64_t> generation{0};   // bumped by edits that move device buffers
   // free cubes (vt_internal.h), built by the first render of the scene
