@@ -46,8 +46,13 @@ VT_API int vt_diag_render_counted(vt_job* job, int32_t passes, uint64_t* counter
                                   int32_t* result);
 
 /* Kernel form used by vt_job_render and vt_render_batch when their options
- * do not say: 1 = plain (one thread per pixel, one launch per pass),
- * 2 = wavefront (path slots over all jobs' work items). */
+ * do not say: 0 (the default) = by the launch's size (a thread per sample up
+ * to 2^17 samples; then wavefronts inside thread blocks, one kernel a launch,
+ * while samples times max_bounces + 2 is at most 2^24; then the wavefront),
+ * 1 = plain (one thread per pixel, one launch per pass), 2 = wavefront (path
+ * slots over all jobs' work items) for every size.  Results are identical.
+ * The wavefront's settings below do not touch the two other forms, except
+ * trace_steps, which the block wavefronts use too. */
 VT_API int vt_diag_set_kernel(vt_context* ctx, int32_t kernel);
 
 /* Wavefront rounds replayed as a captured CUDA graph (enabled = 1, the
@@ -74,11 +79,13 @@ VT_API int vt_diag_cdf_from_function(vt_context* ctx, const float* func, int32_t
 
 /* Tuning of the wavefront form (path_slots, trace_steps and max_items <= 0
  * and trace_blocks_per_sm < 0 keep their value):
- * path_slots paths in flight per launch (default 2M), trace_blocks_per_sm
+ * path_slots paths in flight per launch (default 8M), trace_blocks_per_sm
  * resident blocks of the DDA kernel (0: occupancy limit, the default),
- * trace_steps DDA steps between ray-pool refills (4, 8, 16 or 32; by default
- * 16, 8 where a volume has free cubes),
+ * trace_steps DDA steps between ray-pool refills (4, 8, 16 or 32; by default,
+ * and again after VT_DIAG_TRACE_STEPS_AUTO, 16, or 8 where a volume has free
+ * cubes),
  * max_items samples per launch (sample-buffer entries, default 2^28). */
+#define VT_DIAG_TRACE_STEPS_AUTO (-2147483647 - 1)
 VT_API int vt_diag_set_tuning(vt_context* ctx, int64_t path_slots, int32_t trace_blocks_per_sm,
                               int32_t trace_steps, int64_t max_items);
 

@@ -1,0 +1,63 @@
+"""The wavefront's own forms, asked for by name (kernel 2) whatever a launch's
+size would choose, with the number of kernels launched as the evidence of the
+form: groups of rounds launched directly or replayed, lanes, DDA kernel forms;
+and the way back to a context's defaults."""
+import numpy as np
+import pytest
+
+from helpers import close_all, gpu_setup, small_config2
+from voxeltoy_gb300 import Context, Job, Scene
+from voxeltoy_gb300 import _lib as L
+from voxeltoy_gb300 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def wctx():
+    c = Context()
+    yield c
+    c.close()
+
+
+def config(w, h, bounces=8, edge=24, seed=15):
+    cfg = small_config2(edge=edge, w=w, h=h, seed=seed)
+    cfg.settings.max_samples = 1 << 20
+    cfg.settings.max_bounces = bounces
+    return cfg
+
+
+def frame(ctx, job, passes, **kw):
+    """The image's words and the kernels launched for it."""
+    job.reset()
+    n = ctx.launch_count()
+    ctx.render_batch([job], passes, kernel=2, **kw)
+    n = ctx.launch_count() - n
+    return job.readback().view(np.uint32).copy(), n
+
+
+def group(lanes, rounds):
+    return lanes * rounds * 4      # shade, hit, regen and trace, a lane and round
+
+
+def test_back_to_the_defaults(wctx):
+    """The kernel form and the DDA steps return to the choice by size and by
+    volume; other values are refused."""
+    scene, env, job = gpu_setup(wctx, config(32, 32))
+    try:
+        images = []
+        for kernel, kernels in ((0, 1), (1, 1), (2, group(1, 10) + 1), (0, 1)):
+            wctx.set_kernel(kernel)
+            wctx.set_tuning(trace_steps=32 if kernel else L.VT_DIAG_TRACE_STEPS_AUTO)
+            job.reset()
+            n = wctx.launch_count()
+            job.render(1)
+            assert wctx.launch_count() - n == kernels
+            images.append(job.readback().view(np.uint32).copy())
+        for a in images[1:]:
+            assert np.array_equal(a, images[0])
+        for bad in (-1, 3):
+            with pytest.raises(L.VtError):
+                wctx.set_kernel(bad)
+    finally:
+        close_all(job, scene, env)

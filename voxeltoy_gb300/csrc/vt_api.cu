@@ -2222,7 +2222,7 @@ extern "C" int vt_diag_set_graphs(vt_context* ctx, int32_t enabled) {
 }
 
 extern "C" int vt_diag_set_kernel(vt_context* ctx, int32_t kernel) {
-  VT_CHECK_ARG(ctx && (kernel == 1 || kernel == 2), "kernel must be 1 (plain) or 2 (wavefront)");
+  VT_CHECK_ARG(ctx && kernel >= 0 && kernel <= 2, "kernel must be 0 (by size), 1 (plain) or 2 (wavefront)");
   ctx->kernel = kernel;
   return VT_OK;
 }
@@ -2376,6 +2376,7 @@ extern "C" int vt_diag_set_tuning(vt_context* ctx, int64_t slots, int32_t blocks
   VT_CHECK_ARG(ctx, "context is null");
   if (slots > 0) ctx->max_slots = std::max<int64_t>(32, std::min<int64_t>(slots, (int64_t)1 << 26));
   if (blocks_per_sm >= 0) ctx->trace_blocks_per_sm = blocks_per_sm;
+  if (steps == VT_DIAG_TRACE_STEPS_AUTO) ctx->trace_steps = 0;
   if (steps > 0) ctx->trace_steps = steps <= 4 ? 4 : (steps <= 8 ? 8 : (steps <= 16 ? 16 : 32));
   if (max_items > 0) ctx->max_items = std::max<int64_t>(1024, max_items);
   return VT_OK;

@@ -82,7 +82,8 @@ class Context:
 
     def set_tuning(self, path_slots: int = 0, trace_blocks_per_sm: int = -1, trace_steps: int = 0,
                    max_items: int = 0):
-        """Wavefront launch parameters; 0 (or -1 for trace_blocks_per_sm) keeps a value."""
+        """Wavefront launch parameters; 0 (or -1 for trace_blocks_per_sm) keeps a
+        value, trace_steps = VT_DIAG_TRACE_STEPS_AUTO goes back to the default."""
         L.call("vt_diag_set_tuning", self.h, path_slots, trace_blocks_per_sm, trace_steps, max_items)
 
     def set_trace_tuning(self, queue_chunk: int = 0, refill_min: int = -1):
@@ -107,6 +108,7 @@ class Context:
         return g.value
 
     def set_kernel(self, kernel: int):
+        """Kernel form: 0 by the launch's size (the default), 1 plain, 2 wavefront."""
         L.call("vt_diag_set_kernel", self.h, kernel)
 
     def set_lanes(self, lanes: int):
