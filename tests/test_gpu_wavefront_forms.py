@@ -40,6 +40,23 @@ def group(lanes, rounds):
     return lanes * rounds * 4      # shade, hit, regen and trace, a lane and round
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 3, 4])
+@pytest.mark.parametrize("w,h,passes", [(641, 479, 1), (641, 479, 3), (150, 131, 1), (256, 256, 2)])
+def test_samples_with_a_slot_each_take_one_group(wctx, lanes, w, h, passes):
+    """Launches whose samples all fit the path slots run max_bounces + 2 rounds
+    (made even) once, whatever the sample count leaves when divided by the lanes."""
+    scene, env, job = gpu_setup(wctx, config(w, h))
+    try:
+        wctx.set_lanes(lanes)
+        got, n = frame(wctx, job, passes)
+        assert n == group(lanes, 10) + 1
+        job.reset()
+        wctx.render_batch([job], passes, kernel=1)
+        assert np.array_equal(got, job.readback().view(np.uint32))
+    finally:
+        close_all(job, scene, env)
+
+
 def test_back_to_the_defaults(wctx):
     """The kernel form and the DDA steps return to the choice by size and by
     volume; other values are refused."""
