@@ -57,6 +57,61 @@ def test_samples_with_a_slot_each_take_one_group(wctx, lanes, w, h, passes):
         close_all(job, scene, env)
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 3, 4])
+def test_replayed_groups_equal_direct_ones(wctx, lanes):
+    """Rounds replayed from a graph against the same rounds launched one by one,
+    with fewer slots than samples, so that both take several groups."""
+    scene, env, job = gpu_setup(wctx, config(96, 80))
+    try:
+        wctx.set_lanes(lanes)
+        images, counts = [], []
+        for graphs in (True, False, True):
+            wctx.set_graphs(graphs)
+            a, n = frame(wctx, job, 5, path_slots=4096)
+            images.append(a)
+            counts.append(n)
+        assert counts[0] == counts[1] == counts[2] > 2 * group(lanes, 8)
+        assert np.array_equal(images[0], images[1]) and np.array_equal(images[0], images[2])
+    finally:
+        close_all(job, scene, env)
+
+
+def test_lanes_agree(wctx):
+    scene, env, job = gpu_setup(wctx, config(96, 80))
+    try:
+        images = []
+        for lanes in (1, 2, 3, 4):
+            wctx.set_lanes(lanes)
+            for slots, rounds in ((0, 10), (4096, 8)):
+                a, n = frame(wctx, job, 3, path_slots=slots)
+                assert (n - 1) % group(lanes, rounds) == 0
+                images.append(a)
+        for a in images[1:]:
+            assert np.array_equal(a, images[0])
+    finally:
+        close_all(job, scene, env)
+
+
+@pytest.mark.parametrize("slots", [0, 4096])
+@pytest.mark.parametrize("open_scene", [False, True])
+def test_trace_forms_agree(wctx, slots, open_scene):
+    cfg = config(96, 80)
+    if open_scene:
+        cfg.voxels = np.zeros((96, 90, 84), np.uint8)
+        cfg.voxels[10:14, ::7, ::5] = 1
+    scene, env, job = gpu_setup(wctx, cfg)
+    try:
+        images = []
+        for form in (0, 1):
+            wctx.set_trace_form(form)
+            for steps in (4, 8, 16):
+                wctx.set_tuning(trace_steps=steps)
+                images.append(frame(wctx, job, 3, path_slots=slots)[0])
+        for a in images[1:]:
+            assert np.array_equal(a, images[0])
+    finally:
+        close_all(job, scene, env)
+
 def test_back_to_the_defaults(wctx):
     """The kernel form and the DDA steps return to the choice by size and by
     volume; other values are refused."""
