@@ -11,62 +11,68 @@ namespace vt {
 
 // ------------------------------------------------------------- bit-bricks
 // One thread per brick of the padded brick grid (one border brick on every
-// side), a warp along x, blocks of eight rows, grid y over brick slices.
+// side), in the array's order.
 // Voxels outside the volume read as occupied, so the DDA stops on the first
 // voxel beyond the volume without a separate bounds test.
 //
 // With `max_entry`, the largest palette entry of the volume is atomically
 // max-ed into *max_entry (the host checks it against the palette size).
 // Bound by the read of the volume; border bricks are written without a look
-// at their voxels and indices take no division (a thread per brick of the
-// flattened array, with both, took 30 us for 256^3, now 21).
-constexpr int kBrickRows = 8;
-__global__ void __launch_bounds__(32 * kBrickRows) k_build_bricks(const uint8_t* __restrict__ grid, int32_t rx,
-                                                                  int32_t ry, int32_t rz,
-                                                                  unsigned long long* __restrict__ bricks, int32_t bx,
-                                                                  int32_t by, int32_t bz, const BrickShape sh,
-                                                                  unsigned long long* max_entry) {
-  const int px = bx + 2, py = by + 2;
-  const int iy = blockIdx.x * kBrickRows + threadIdx.y;
+// at their voxels, and the indices (below 2^32 bricks) take two high
+// multiplies.  Call with allocation and wait, us: 256^3, 1024^3 and 1048574x1x1
+// with 64-bit divisions and every voxel of the border looked at 41, 699 and
+// 184; without, a warp to a row and eight rows a block, whose reads lie further
+// apart and which leaves a volume along x to a few warps, 27, 840 and 15294;
+// now 22, 553 and 36.
+constexpr int kBrickThreads = 256;
+__global__ void __launch_bounds__(kBrickThreads) k_build_bricks(const uint8_t* __restrict__ grid, int32_t rx,
+                                                                int32_t ry, int32_t rz,
+                                                                unsigned long long* __restrict__ bricks, int32_t bx,
+                                                                int32_t by, int32_t bz, uint64_t m_px, uint64_t m_pxy,
+                                                                const BrickShape sh, unsigned long long* max_entry) {
+  const uint32_t px = bx + 2, pxy = px * (uint32_t)(by + 2);
+  const uint32_t b = blockIdx.x * kBrickThreads + threadIdx.x;
   unsigned top = 0;
-  for (int iz = blockIdx.y; iz < bz + 2; iz += gridDim.y)
-    for (int ix = threadIdx.x; ix < px && iy < py; ix += 32) {
-      unsigned long long w = 0ull;
-      const int ex = 1 << sh.sx, ey = 1 << sh.sy, ez = 1 << sh.sz;
-      const int x0 = (ix - 1) * ex, y0 = (iy - 1) * ey, z0 = (iz - 1) * ez;
-      if (ix == 0 || iy == 0 || iz == 0 || ix > bx || iy > by || iz > bz) {
-        w = ~0ull;   // border
-      } else if (sh.sx == 2 && sh.sy == 2 && (rx & 3) == 0) {
-        // 4x4x4 bricks: rows of four voxels as one aligned 32-bit word where
-        // rows start on 4-byte boundaries; the sixteen loads are independent
-        unsigned tops = 0u;   // byte-wise maximum of the word rows
+  const int iz = (int)udiv(b, m_pxy);
+  if (iz < bz + 2) {
+    const uint32_t r = b - (uint32_t)iz * pxy;
+    const int iy = (int)udiv(r, m_px), ix = (int)(r - (uint32_t)iy * px);
+    unsigned long long w = 0ull;
+    const int ex = 1 << sh.sx, ey = 1 << sh.sy, ez = 1 << sh.sz;
+    const int x0 = (ix - 1) * ex, y0 = (iy - 1) * ey, z0 = (iz - 1) * ez;
+    if (ix == 0 || iy == 0 || iz == 0 || ix > bx || iy > by || iz > bz) {
+      w = ~0ull;   // border
+    } else if (sh.sx == 2 && sh.sy == 2 && (rx & 3) == 0) {
+      // 4x4x4 bricks: rows of four voxels as one aligned 32-bit word where
+      // rows start on 4-byte boundaries; the sixteen loads are independent
+      unsigned tops = 0u;   // byte-wise maximum of the word rows
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-          const int y = y0 + (r & 3), z = z0 + (r >> 2);
-          const bool in = y < ry && z < rz;
-          const uint32_t v4 =
-              in ? *reinterpret_cast<const uint32_t*>(grid + (size_t)x0 + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z))
-                 : 0u;
-          tops = __vmaxu4(tops, v4);
-          uint32_t m = __vcmpne4(v4, 0u) & 0x01010101u;   // bit 0 of each non-zero byte
-          m = (m | (m >> 7) | (m >> 14) | (m >> 21)) & 0xfu;
-          w |= (unsigned long long)(in ? m : 0xfu) << (4 * r);   // rows outside the volume read as set
-        }
-        for (int k = 0; k < 32; k += 8) top = max(top, (tops >> k) & 0xffu);
-      } else {
-        for (int k = 0; k < 64; ++k) {
-          const int x = x0 + (k & (ex - 1)), y = y0 + ((k >> sh.sx) & (ey - 1)), z = z0 + (k >> (sh.sx + sh.sy));
-          const bool outside = x >= rx || y >= ry || z >= rz;
-          const unsigned v = outside ? 0u : grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)];
-          top = v > top ? v : top;
-          if (outside || v != 0) w |= 1ull << k;
-        }
+      for (int r = 0; r < 16; ++r) {
+        const int y = y0 + (r & 3), z = z0 + (r >> 2);
+        const bool in = y < ry && z < rz;
+        const uint32_t v4 =
+            in ? *reinterpret_cast<const uint32_t*>(grid + (size_t)x0 + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z))
+               : 0u;
+        tops = __vmaxu4(tops, v4);
+        uint32_t m = __vcmpne4(v4, 0u) & 0x01010101u;   // bit 0 of each non-zero byte
+        m = (m | (m >> 7) | (m >> 14) | (m >> 21)) & 0xfu;
+        w |= (unsigned long long)(in ? m : 0xfu) << (4 * r);   // rows outside the volume read as set
       }
-      bricks[(int64_t)ix + (int64_t)px * ((int64_t)iy + (int64_t)py * iz)] = w;
+      for (int k = 0; k < 32; k += 8) top = max(top, (tops >> k) & 0xffu);
+    } else {
+      for (int k = 0; k < 64; ++k) {
+        const int x = x0 + (k & (ex - 1)), y = y0 + ((k >> sh.sx) & (ey - 1)), z = z0 + (k >> (sh.sx + sh.sy));
+        const bool outside = x >= rx || y >= ry || z >= rz;
+        const unsigned v = outside ? 0u : grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)];
+        top = v > top ? v : top;
+        if (outside || v != 0) w |= 1ull << k;
+      }
     }
+    bricks[b] = w;
+  }
   // an atomic only where it would raise the maximum
   top = __reduce_max_sync(0xffffffffu, top);
-  if (max_entry && threadIdx.x == 0 && top > *(volatile unsigned long long*)max_entry)
+  if (max_entry && (threadIdx.x & 31) == 0 && top > *(volatile unsigned long long*)max_entry)
     atomicMax(max_entry, (unsigned long long)top);
 }
 
@@ -346,8 +352,10 @@ cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t 
 cudaError_t launch_build_bricks(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
                                 unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, const BrickShape& sh,
                                 unsigned long long* max_entry, cudaStream_t st) {
-  const dim3 blocks((unsigned)((by + 2 + kBrickRows - 1) / kBrickRows), (unsigned)std::min(bz + 2, 65535));
-  k_build_bricks<<<blocks, dim3(32, kBrickRows), 0, st>>>(grid, rx, ry, rz, bricks, bx, by, bz, sh, max_entry);
+  const uint32_t px = bx + 2, pxy = px * (uint32_t)(by + 2);
+  const int64_t n = (int64_t)pxy * (bz + 2);
+  k_build_bricks<<<(unsigned)((n + kBrickThreads - 1) / kBrickThreads), kBrickThreads, 0, st>>>(
+      grid, rx, ry, rz, bricks, bx, by, bz, udiv_magic(px), udiv_magic(pxy), sh, max_entry);
   return cudaGetLastError();
 }
 
