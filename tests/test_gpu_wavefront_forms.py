@@ -133,3 +133,33 @@ def test_back_to_the_defaults(wctx):
                 wctx.set_kernel(bad)
     finally:
         close_all(job, scene, env)
+
+@pytest.mark.parametrize("w,h,inside,block", [(512, 512, True, True), (513, 512, True, False), (513, 512, False, True),
+                                              (480, 270, True, True)])
+def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, inside, block):
+    """A launch by size takes one kernel and the accumulation (a single pass of
+    few samples one kernel), or the wavefront's; the images are the same."""
+    cfg = config(w, h, bounces=3)
+    if inside:
+        cfg.voxels = np.ones((24, 24, 24), np.uint8)
+        cfg.voxels[3:-3, 3:-3, 3:-3] = 0
+        cfg.voxels[20, 21, 10:14] = 2
+        cfg.camera = S.orbit_camera(distance=150.0)
+    scene, env, job = gpu_setup(wctx, cfg)
+    other = Job(wctx, scene, env, cfg.camera, cfg.settings, 40, 30)
+    try:
+        want, rounds = frame(wctx, job, 1)
+        job.reset()
+        n = wctx.launch_count()
+        job.render(1)
+        n = wctx.launch_count() - n
+        assert n == ((1 if w * h <= 1 << 17 else 2) if block else rounds)
+        assert np.array_equal(job.readback().view(np.uint32), want)
+        job.reset()
+        n = wctx.launch_count()
+        wctx.render_batch([job, other], 1)            # both cameras count
+        n = wctx.launch_count() - n
+        assert n == (2 if not inside or w * h + 1200 <= 1 << 18 else rounds)
+        assert np.array_equal(job.readback().view(np.uint32), want)
+    finally:
+        close_all(other, job, scene, env)
