@@ -2022,11 +2022,8 @@ extern "C" int vt_scene_set_voxel(vt_scene* s, int32_t x, int32_t y, int32_t z, 
   // server's first render of the scene) see it, or are there to be lowered
   std::lock_guard<std::mutex> g(s->runs_mu);
   const int64_t idx = (int64_t)x + (int64_t)s->res[0] * ((int64_t)y + (int64_t)s->res[1] * z);
-  VT_CUDA(launch_set_voxel(s->grid, s->bricks, s->res[0], s->res[1], s->bdim[0], s->bdim[1], scene_shape(s), x, y,
-                           z, (uint8_t)entry, ctx->stream), "voxel edit");
-  if (entry && s->runs.load())
-    VT_CUDA(launch_free_cubes_edit(s->runs.load(), s->bdim[0], s->bdim[1], s->bdim[2], x >> 2, y >> 2, z >> 2,
-                                   ctx->stream), "voxel edit");
+  VT_CUDA(launch_set_voxel(s->grid, s->bricks, s->res[0], s->res[1], s->bdim[0], s->bdim[1], s->bdim[2], scene_shape(s),
+                           x, y, z, (uint8_t)entry, s->runs.load(), ctx->stream), "voxel edit");
   int rc = VT_OK;
   if (s->flags & VT_SCENE_AUTO_EMISSIVE) {
     rc = scene_emissive(ctx, s, nullptr, 0, s->flags);          // rediscover from the palette

@@ -158,8 +158,10 @@ cudaError_t launch_l2_read(const uint4* buf, uint32_t n, int32_t reps, uint4* ou
 cudaError_t read_check_word(uint32_t* word, bool* enabled, bool reset);
 
 // ---- scene (vt_scene.cu)
+// runs (nullable): the scene's free cubes, lowered around a voxel that is set.
 cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t rx, int32_t ry, int32_t bx, int32_t by,
-                             const BrickShape& sh, int32_t x, int32_t y, int32_t z, uint8_t entry, cudaStream_t st);
+                             int32_t bz, const BrickShape& sh, int32_t x, int32_t y, int32_t z, uint8_t entry,
+                             unsigned long long* runs, cudaStream_t st);
 // max_entry (nullable): receives the largest palette entry of the volume.
 cudaError_t launch_build_bricks(const uint8_t* grid, int32_t rx, int32_t ry, int32_t rz,
                                 unsigned long long* bricks, int32_t bx, int32_t by, int32_t bz, const BrickShape& sh,
@@ -173,9 +175,6 @@ cudaError_t launch_free_cubes_open(const unsigned long long* bricks, int32_t bx,
                                    uint32_t** open, int sm_count, cudaStream_t st);
 cudaError_t launch_free_cubes(int32_t bx, int32_t by, int32_t bz, void* scratch, unsigned long long* runs,
                               cudaStream_t st);
-// After brick (x, y, z) became occupied.
-cudaError_t launch_free_cubes_edit(unsigned long long* runs, int32_t bx, int32_t by, int32_t bz, int32_t x, int32_t y,
-                                   int32_t z, cudaStream_t st);
 // A volume as the emissive passes see it.
 struct EmissiveVolume {
   int32_t rx, ry, rz;

@@ -315,10 +315,9 @@ cudaError_t launch_free_cubes(int32_t bx, int32_t by, int32_t bz, void* scratch,
 // before it.  One thread per brick within reach; a brick that became empty
 // leaves them as they are, still lower bounds.
 constexpr int kReach = 2 * kMaxFreeCube - 1;
-__global__ void k_cubes_edit(unsigned long long* runs, int32_t px, int32_t py, int32_t pz, int32_t x, int32_t y,
-                             int32_t z) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kReach * kReach * kReach) return;
+constexpr int kReachBricks = kReach * kReach * kReach;
+__device__ __forceinline__ void cubes_edit(int i, unsigned long long* runs, int32_t px, int32_t py, int32_t pz, int32_t x,
+                                           int32_t y, int32_t z) {
   const int ox = i % kReach - (kMaxFreeCube - 1), oy = (i / kReach) % kReach - (kMaxFreeCube - 1),
             oz = i / (kReach * kReach) - (kMaxFreeCube - 1);
   const int vx = x - ox, vy = y - oy, vz = z - oz;   // the edited brick lies (ox, oy, oz) from this one
@@ -336,27 +335,30 @@ __global__ void k_cubes_edit(unsigned long long* runs, int32_t px, int32_t py, i
   *at = w;
 }
 
-cudaError_t launch_free_cubes_edit(unsigned long long* runs, int32_t bx, int32_t by, int32_t bz, int32_t x, int32_t y,
-                                   int32_t z, cudaStream_t st) {
-  const int n = kReach * kReach * kReach;
-  k_cubes_edit<<<(n + 127) / 128, 128, 0, st>>>(runs, bx + 2, by + 2, bz + 2, x + 1, y + 1, z + 1);
-  return cudaGetLastError();
-}
-
-// One voxel edit: its grid entry and its bit in the padded brick grid.
+// One voxel edit: its grid entry and its bit in the padded brick grid, and with
+// `runs` the free cubes around its brick, in the same launch (a second one made
+// an edit of a scene with free cubes 10.5 -> 12.3 us).
 __global__ void k_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t rx, int32_t ry, int32_t bx, int32_t by,
-                            const BrickShape sh, int32_t x, int32_t y, int32_t z, uint8_t entry) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)] = entry;
-  const int64_t b = brick_index_of(sh, bx, by, x, y, z);
-  const unsigned long long bit = 1ull << brick_bit_of(sh, x, y, z);
-  if (entry) atomicOr(&bricks[b], bit);
-  else atomicAnd(&bricks[b], ~bit);
+                            int32_t bz, const BrickShape sh, int32_t x, int32_t y, int32_t z, uint8_t entry,
+                            unsigned long long* runs) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    grid[(size_t)x + (size_t)rx * ((size_t)y + (size_t)ry * (size_t)z)] = entry;
+    const int64_t b = brick_index_of(sh, bx, by, x, y, z);
+    const unsigned long long bit = 1ull << brick_bit_of(sh, x, y, z);
+    if (entry) atomicOr(&bricks[b], bit);
+    else atomicAnd(&bricks[b], ~bit);
+  }
+  if (runs && i < kReachBricks)   // 4x4x4 bricks
+    cubes_edit(i, runs, bx + 2, by + 2, bz + 2, (x >> 2) + 1, (y >> 2) + 1, (z >> 2) + 1);
 }
 
 cudaError_t launch_set_voxel(uint8_t* grid, unsigned long long* bricks, int32_t rx, int32_t ry, int32_t bx, int32_t by,
-                             const BrickShape& sh, int32_t x, int32_t y, int32_t z, uint8_t entry, cudaStream_t st) {
-  k_set_voxel<<<1, 32, 0, st>>>(grid, bricks, rx, ry, bx, by, sh, x, y, z, entry);
+                             int32_t bz, const BrickShape& sh, int32_t x, int32_t y, int32_t z, uint8_t entry,
+                             unsigned long long* runs, cudaStream_t st) {
+  if (!entry) runs = nullptr;
+  const int threads = runs ? 128 : 32, blocks = runs ? (kReachBricks + threads - 1) / threads : 1;
+  k_set_voxel<<<blocks, threads, 0, st>>>(grid, bricks, rx, ry, bx, by, bz, sh, x, y, z, entry, runs);
   return cudaGetLastError();
 }
 
