@@ -69,14 +69,16 @@ __global__ void __launch_bounds__(128) k_plain(const Frame F, const JobDev J, in
 
 // The edit-mode integrator by itself: a warp takes a tile of 8 x per_warp / 8
 // pixels.  What bounds it is the latency of the longest rays' dependent brick
-// reads.  Without the path tracer's code it fits in a third of k_plain's 128
-// registers, so that a 512^2 image's warps are all resident at once instead of
-// in four turns, and the rays of a tile end closer together than those of a
-// row.  A 1.3 M-triangle mesh into 1024^3 and its first 512^2 image: 1187 ->
-// 1140 us; at eight resident blocks, without the spills, the same, in rows of
-// 32 pixels 17 us more.
+// reads, and the instructions between them.  Without the path tracer's code it
+// fits in half of k_plain's 128 registers, so that a 512^2 image's warps run in
+// two turns instead of four, and the rays of a tile end closer together than
+// those of a row.  Eight resident blocks, without spills; at twelve, with 64
+// bytes of them, more warps run at once and every image is slower: a 1.3
+// M-triangle mesh into 1024^3 and its first 512^2 image 1017 us against 982, 8
+// passes of 512^2 of 128^3 noise 355 against 315 (541 in k_plain), a 160x120
+// view inside a 48^3 room 36.1 us against 31.8 (34.5).
 template <bool kCount>
-__global__ void __launch_bounds__(128, 12) k_edit(const Frame F, const JobDev J, int sample_base, int passes,
+__global__ void __launch_bounds__(128, 8) k_edit(const Frame F, const JobDev J, int sample_base, int passes,
                                                   int per_warp, int tiles_x, unsigned long long* counters) {
   Cnt<kCount> cnt;
 #pragma unroll
