@@ -163,3 +163,20 @@ def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, insi
         assert np.array_equal(job.readback().view(np.uint32), want)
     finally:
         close_all(other, job, scene, env)
+
+def test_tuning_times_the_wavefront_and_leaves_the_form(wctx):
+    """A small job's sweep launches wavefronts; afterwards its renders take the
+    form by size again."""
+    from voxeltoy_gb300 import autotune
+    scene, env, job = gpu_setup(wctx, config(32, 32))
+    try:
+        n = wctx.launch_count()
+        best = autotune.tune(wctx, [job], passes=1, repeats=1, use_cache=False,
+                             grid={"path_slots": [1 << 20], "trace_blocks_per_sm": [0], "trace_steps": [8, 16],
+                                   "lanes": [1], "brick_shape": [(2, 2, 2)], "queue_chunk": [64], "refill_min": [0]})
+        assert wctx.launch_count() - n >= (group(1, 10) + 1) * len(best["sweep"]) * best["repeats"]
+        n = wctx.launch_count()
+        job.render(1)
+        assert wctx.launch_count() - n == 1
+    finally:
+        close_all(job, scene, env)

@@ -17,11 +17,15 @@ and last the pooled form of the DDA kernel (segment set-up for a warp's
 worth of records at once, lanes refilled from a shared-memory pool) at
 trace_form_steps steps per batch.
 and applies the fastest setting to the context.  Every setting renders the
-same bits.  Path-slot counts above the workload's samples collapse to one
-setting; frames shorter than a few milliseconds are timed several times per
-setting.  Results are cached in a JSON file keyed by a workload class (log2
-of the largest grid edge, log2 of the pixels per pass, number of jobs) and
-the set of knobs swept, so later runs with a similar workload skip the sweep.
+same bits.  The timed renders are wavefront launches whatever their size: the
+forms that launches of few samples take by themselves read none of the knobs
+but trace_steps, and a pick among equal times would be noise, applied to larger
+renders later.  The context's own choice of form is put back after the sweep.
+Path-slot counts above the workload's samples collapse to one setting; frames
+shorter than a few milliseconds are timed several times per setting.  Results
+are cached in a JSON file keyed by a workload class (log2 of the largest grid
+edge, of the pixels per pass and of the samples timed, number of jobs) and the
+set of knobs swept, so later runs with a similar workload skip the sweep.
 """
 from __future__ import annotations
 
@@ -38,11 +42,14 @@ DEFAULT_GRID = {
     "trace_steps": [8, 16, 32],
     "lanes": [2, 3, 1],
     "brick_shape": [(2, 2, 2), (3, 2, 1), (1, 3, 2), (2, 1, 3)],
-    "queue_chunk": [128, 64, 256],
+    "queue_chunk": [64, 128, 256],
     "refill_min": [0, 12, 20],
     "trace_form_steps": [8, 16],
 }
-KNOBS = "slots,bps,steps,lanes,brick,chunk,refill,form"
+# The knobs and what they were timed on (the wavefront, whose DDA kernel leaps
+# through the free cubes of 4x4x4 bricks): picks made for others do not apply.
+KNOBS = "slots,bps,steps,lanes,brick,chunk,refill,form,wavefront,leaps"
+WAVEFRONT = 2   # Context.set_kernel
 
 
 def cache_path() -> Path:
@@ -52,17 +59,19 @@ def cache_path() -> Path:
     return Path.home() / ".cache" / "voxeltoy_gb300" / "tune.json"
 
 
-def workload_key(jobs) -> str:
+def workload_key(jobs, passes: int = 16) -> str:
+    def log2(n):
+        return int(round(math.log2(max(n, 1))))
+
     edge = max(max(j.scene.info().resolution) for j in jobs)
     pixels = sum(j.width * j.height for j in jobs)
-    return (f"edge{int(round(math.log2(max(edge, 1))))}_px{int(round(math.log2(max(pixels, 1))))}_jobs{len(jobs)}"
-            f"_{KNOBS}")
+    return f"edge{log2(edge)}_px{log2(pixels)}_samples{log2(pixels * passes)}_jobs{len(jobs)}_{KNOBS}"
 
 
 def _apply(ctx, setting: dict, jobs=()):
     ctx.set_lanes(setting.get("lanes", 2))
     ctx.set_tuning(setting["path_slots"], setting["trace_blocks_per_sm"], setting["trace_steps"])
-    ctx.set_trace_tuning(setting.get("queue_chunk", 128), setting.get("refill_min", 0))
+    ctx.set_trace_tuning(setting.get("queue_chunk", 64), setting.get("refill_min", 0))
     if hasattr(ctx, "set_trace_form"):
         ctx.set_trace_form(setting.get("trace_form", 0))
     shape = tuple(setting.get("brick_shape", (2, 2, 2)))
@@ -89,25 +98,9 @@ def _time_render(ctx, jobs, passes: int, repeats: int) -> float:
     return best
 
 
-def tune(ctx, jobs, passes: int = 16, repeats: int = 2, grid: dict | None = None, use_cache: bool = True) -> dict:
-    """Sweep the grid on `passes` samples per pixel of `jobs`, apply and return
-    the best setting ({"path_slots", "trace_blocks_per_sm", "trace_steps",
-    "lanes", "seconds", "key", "cached"}).  `grid` overrides entries of
-    DEFAULT_GRID."""
-    key = workload_key(jobs)
-    path = cache_path()
-    cache = {}
-    if use_cache and path.exists():
-        try:
-            cache = json.loads(path.read_text())
-        except (OSError, ValueError):
-            cache = {}
-    if use_cache and key in cache:
-        best = dict(cache[key])
-        _apply(ctx, best, jobs)
-        best.update(key=key, cached=True)
-        return best
-    grid = dict(DEFAULT_GRID, **(grid or {}))
+def _sweep(ctx, jobs, passes: int, repeats: int, grid: dict):
+    """Every (seconds, setting) timed, the best of them, and the renders timed
+    for each."""
     items = passes * sum(j.width * j.height for j in jobs)
     slot_list = sorted({min(s, max(items, 32)) for s in grid["path_slots"]})
     _apply(ctx, {"path_slots": slot_list[-1], "trace_blocks_per_sm": 0, "trace_steps": 16})
@@ -147,7 +140,35 @@ def tune(ctx, jobs, passes: int = 16, repeats: int = 2, grid: dict | None = None
         _apply(ctx, setting, jobs)
         final.append((_time_render(ctx, jobs, passes, 3 * reps), setting))
     final.sort(key=lambda r: r[0])
-    t, best = final[0]
+    return results, final[0], reps
+
+
+def tune(ctx, jobs, passes: int = 16, repeats: int = 2, grid: dict | None = None, use_cache: bool = True) -> dict:
+    """Sweep the grid on `passes` samples per pixel of `jobs`, apply and return
+    the best setting ({"path_slots", "trace_blocks_per_sm", "trace_steps",
+    "lanes", "seconds", "key", "cached"}).  `grid` overrides entries of
+    DEFAULT_GRID."""
+    key = workload_key(jobs, passes)
+    path = cache_path()
+    cache = {}
+    if use_cache and path.exists():
+        try:
+            cache = json.loads(path.read_text())
+        except (OSError, ValueError):
+            cache = {}
+    if use_cache and key in cache:
+        best = dict(cache[key])
+        _apply(ctx, best, jobs)
+        best.update(key=key, cached=True)
+        return best
+    kernel = getattr(ctx, "kernel", None)
+    if kernel is not None:
+        ctx.set_kernel(WAVEFRONT)
+    try:
+        results, (t, best), reps = _sweep(ctx, jobs, passes, repeats, dict(DEFAULT_GRID, **(grid or {})))
+    finally:
+        if kernel is not None:
+            ctx.set_kernel(kernel)
     _apply(ctx, best, jobs)
     best = dict(best, seconds=t)
     for j in jobs:

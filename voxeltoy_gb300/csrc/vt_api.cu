@@ -1681,10 +1681,10 @@ static int wf_launch(vt_context* ctx, std::vector<JobEntry>& entries, const std:
   int lanes = ctx->lanes;
   while (lanes > 1 && (items < 4096 * (int64_t)lanes || slots < 1024 * (int64_t)lanes)) --lanes;
   const int64_t lane_items = items - items / lanes * (lanes - 1);
-  // a slot for every sample of the largest share where the cap allows them,
-  // whatever the division leaves (641x479 x 14 samples of 128^3 noise, 25 of
+  // a slot for every sample of the largest share where the cap allows all
+  // samples in flight, whatever the division leaves (641x479 x 14 samples of 128^3 noise, 25 of
   // them without a slot before: 1974 -> 1631 us, by one group of rounds below)
-  if (lanes > 1 && (lane_items + 31) / 32 * 32 * lanes <= slots_cap) slots = (lane_items + 31) / 32 * 32 * lanes;
+  if (lanes > 1 && items <= slots_cap) slots = (lane_items + 31) / 32 * 32 * lanes;
   const size_t lane_slots = lanes > 1 ? ((size_t)slots / lanes) & ~(size_t)31 : (size_t)slots;   // 256-byte lane bases
   int rc = wf_reserve(ctx, slots, items);
   if (rc != VT_OK) return rc;

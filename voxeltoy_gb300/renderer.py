@@ -46,6 +46,7 @@ class Context:
         h = C.c_void_p()
         L.call("vt_create", C.byref(opts), C.byref(h))
         self.h = h
+        self.kernel = 0            # the form set_kernel chose last
         self._log_cb = None
 
     def close(self):
@@ -110,6 +111,7 @@ class Context:
     def set_kernel(self, kernel: int):
         """Kernel form: 0 by the launch's size (the default), 1 plain, 2 wavefront."""
         L.call("vt_diag_set_kernel", self.h, kernel)
+        self.kernel = kernel
 
     def set_lanes(self, lanes: int):
         """Wavefront lanes side by side on their own streams (1-4; 2 is the default)."""
