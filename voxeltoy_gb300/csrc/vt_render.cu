@@ -129,7 +129,8 @@ __global__ void k_diag(const Frame F, const JobDev J, int sample, float4* out, H
   if (idx < n) {
     const int px = idx % F.width, py = idx / F.width;
     HitRecord h;
-    const float4 v = trace_sample(F, J, px, py, sample, cnt, &h);
+    const float4 v = F.integrator == 1 ? edit_sample(F, J, px, py, sample, cnt, &h)
+                                       : trace_sample(F, J, px, py, sample, cnt, &h);
     out[idx] = v;
     if (hits) hits[idx] = h;
   }

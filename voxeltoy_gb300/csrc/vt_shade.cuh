@@ -1202,7 +1202,6 @@ VT_D float4 edit_sample(const Frame& F, const JobDev& J, int px, int py, int sam
 template <bool kCount>
 VT_D float4 trace_sample(const Frame& F, const JobDev& J, int px, int py, int sample, Cnt<kCount>& cnt,
                          HitRecord* first_hit) {
-  if (F.integrator == 1) return edit_sample(F, J, px, py, sample, cnt, first_hit);
   const Grid g = grid_of(F, J);
   Path p;
   Dda s;
