@@ -134,7 +134,7 @@ def test_back_to_the_defaults(wctx):
     finally:
         close_all(job, scene, env)
 
-@pytest.mark.parametrize("w,h,inside,block", [(512, 512, True, True), (513, 512, True, False), (513, 512, False, True),
+@pytest.mark.parametrize("w,h,inside,block", [(768, 512, True, True), (769, 512, True, False), (769, 512, False, True),
                                               (480, 270, True, True)])
 def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, inside, block):
     """A launch by size takes one kernel and the accumulation (a single pass of
@@ -159,7 +159,7 @@ def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, insi
         n = wctx.launch_count()
         wctx.render_batch([job, other], 1)            # both cameras count
         n = wctx.launch_count() - n
-        assert n == (2 if not inside or w * h + 1200 <= 1 << 18 else rounds)
+        assert n == (2 if not inside or w * h + 1200 <= 3 << 17 else rounds)
         assert np.array_equal(job.readback().view(np.uint32), want)
     finally:
         close_all(other, job, scene, env)

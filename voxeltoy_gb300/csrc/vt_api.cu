@@ -1549,12 +1549,13 @@ constexpr int64_t kBlockWork = 16 << 20;
 // primary rays misses it, and in a closed room every path goes on to
 // max_bounces, so that the rounds are full and the block form's price per
 // segment outweighs the launches.  Block against wavefront, us, four and eight
-// bounces: 128^3 rooms with furniture, 262 k samples 704 / 783 and 1355 / 1446,
+// bounces: a 128^3 room with furniture, 262 k samples 704 / 783 and 1355 / 1446,
 // 393 k 1022 / 919 and 1975 / 1696, 1.05 M 2242 / 1690 and 4348 / 3243; a hollow
-// in 128^3 noise, 262 k 528 / 670 and 849 / 1110, 614 k 1049 / 917 and
-// 1595 / 1487.  Seen from outside, a 64^3 box with its front open, 1.05 M
-// 1144 / 1039 and 1635 / 1578.
-constexpr int64_t kBlockInside = 1 << 18;
+// in 128^3 noise, 393 k 729 / 760 and 1138 / 1257, 614 k 1049 / 917 and
+// 1595 / 1487; an empty 48^3 room, four bounces, 320 k 540 / 636, 614 k 924 / 898.
+// Seen from outside, a 64^3 box with its front open, 1.05 M 1144 / 1039 and
+// 1635 / 1578.
+constexpr int64_t kBlockInside = 3 << 17;
 
 static bool eye_inside(const Frame& F) {
   bool in = true;   // the eye is the translation of the inverse model-view matrix
