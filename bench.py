@@ -754,7 +754,7 @@ def main():
     ap.add_argument("--spp", type=int, default=None, help="samples per pixel (256; 16 for config1)")
     ap.add_argument("--cpu-seconds", type=float, default=16.0)
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
-    ap.add_argument("--kernel", type=int, default=2, help="1 plain per-pass launches, 2 wavefront")
+    ap.add_argument("--kernel", type=int, default=2, help="0 by the launch's size, 1 plain per-pass launches, 2 wavefront")
     ap.add_argument("--no-tune", action="store_true", help="skip the autotuner (library defaults)")
     ap.add_argument("--slots", type=int, default=0, help="path slots per launch (skips the autotuner)")
     ap.add_argument("--lanes", type=int, default=2, choices=[1, 2, 3, 4], help="wavefront lanes with --slots")

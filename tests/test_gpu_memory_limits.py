@@ -20,8 +20,8 @@ def open_volume(edge):
 
 @pytest.mark.parametrize("integrator", [0, 1])
 def test_a_render_goes_on_where_free_cubes_find_no_memory(integrator):
-    """The first render of an open scene on a device without room for its free
-    cubes succeeds without them, and counts its samples."""
+    """The renders of an open scene on a device without room for its free cubes
+    succeed without them, and count their samples."""
     torch = pytest.importorskip("torch")
     vox = open_volume(512)
     cam, s = S.orbit_camera(distance=500.0), S.physical_settings(3, seed=4)
@@ -33,7 +33,8 @@ def test_a_render_goes_on_where_free_cubes_find_no_memory(integrator):
             before = b.info().device_bytes
             for j in jobs:
                 j.set_integrator(integrator)
-            jobs[0].render(1)                      # its kernels are loaded, its buffers there
+            for _ in range(2):                     # its kernels are loaded, its buffers there
+                jobs[0].render(1)
             want = jobs[0].readback()
             jobs[1].readback()
             assert a.info().device_bytes > before
@@ -44,8 +45,9 @@ def test_a_render_goes_on_where_free_cubes_find_no_memory(integrator):
                     held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
                 except torch.cuda.OutOfMemoryError:
                     size //= 2
-            jobs[1].render(1)
-            assert jobs[1].samples() == 1 and b.info().device_bytes == before
+            for _ in range(2):
+                jobs[1].render(1)
+            assert jobs[1].samples() == 2 and b.info().device_bytes == before
             assert np.array_equal(jobs[1].readback().view(np.uint32), want.view(np.uint32))
         finally:
             held.clear()
@@ -98,3 +100,26 @@ def test_device_bytes_count_the_free_cubes():
             assert scene.info().device_bytes == before
         finally:
             close_all(job, scene)
+
+
+@pytest.mark.parametrize("edge,w,h,passes,built", [(96, 64, 48, 1, 2), (96, 1024, 1024, 2, 1), (640, 64, 48, 1, 1)])
+def test_a_first_edit_mode_image_leaves_the_free_cubes_to_the_second(edge, w, h, passes, built):
+    """A scene's first edit-mode image builds free cubes where the volume or the
+    call is large, any other image does, and all are the same without them."""
+    with Context() as ctx:
+        scenes = [Scene.dense(ctx, open_volume(edge), PALETTE) for _ in range(3)]
+        jobs = [Job(ctx, sc, None, S.orbit_camera(distance=700.0), S.physical_settings(2), w, h) for sc in scenes]
+        try:
+            scenes[1].set_brick_shape((1, 2, 3))
+            bytes_ = [sc.info().device_bytes for sc in scenes]
+            for n in (1, 2, 3):
+                for j in jobs[:2]:
+                    j.set_integrator(1)
+                    j.render(passes)
+                assert (scenes[0].info().device_bytes > bytes_[0]) == (n >= built)
+                a, b = (j.readback().view(np.uint32) for j in jobs[:2])
+                assert np.array_equal(a, b)
+            jobs[2].render(1)                              # the path tracer's first image
+            assert scenes[2].info().device_bytes > bytes_[2]
+        finally:
+            close_all(*jobs, *scenes)

@@ -1418,10 +1418,22 @@ static int build_free_cubes(vt_context* ctx, vt_scene* s) {
   return VT_OK;
 }
 
-static int ensure_free_cubes(vt_context* ctx, const vt_scene* scene) {
-  vt_scene* s = const_cast<vt_scene*>(scene);
+// An edit-mode image has one or two segments a sample, so a scene's first one
+// does not make up for the build (two waits, some 55 us) unless the volume or
+// the call is large; another render of the scene builds them.  First 512^2
+// image of a mesh, built / not built: 320^3 (0.55 M padded bricks) 157 / 103 us,
+// 512^3 (2.2 M) 200 / 160, 640^3 (4.3 M) 231 / 221, 800^3 302 / 305; 1920x1080 of
+// 400^3 277 / 266, of 512^3 313 / 337.
+constexpr int64_t kEditBricks = 1 << 22;
+constexpr int64_t kEditSamples = 1 << 21;
+
+static int ensure_free_cubes(vt_context* ctx, const vt_job* j, int passes) {
+  vt_scene* s = const_cast<vt_scene*>(j->scene);
   // without the lock, which an edit holds until its stream is idle
   if (s->runs_tried) return VT_OK;
+  if (j->integrator == VT_INTEGRATOR_EDIT_MODE && (int64_t)j->w * j->h * passes < kEditSamples &&
+      (int64_t)(s->bdim[0] + 2) * (s->bdim[1] + 2) * (s->bdim[2] + 2) < kEditBricks && !s->shown.exchange(true))
+    return VT_OK;
   std::lock_guard<std::mutex> g(s->runs_mu);
   if (s->runs_tried) return VT_OK;
   const int rc = build_free_cubes(ctx, s);
@@ -1450,7 +1462,7 @@ int vt::render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32
   vt::Range nvtx_range("vt.render");
   cudaSetDevice(ctx->device);
   for (int32_t i = 0; i < n; ++i) {
-    int rc = count ? VT_OK : ensure_free_cubes(ctx, jobs[i]->scene);
+    int rc = count ? VT_OK : ensure_free_cubes(ctx, jobs[i], passes[i]);
     if (rc == VT_OK) rc = refresh_job(jobs[i]);
     if (rc != VT_OK) return rc;
   }

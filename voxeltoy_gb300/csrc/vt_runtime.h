@@ -108,9 +108,11 @@ struct vt_scene {
   std::atomic<uint64_t> bytes{0};        // a server's thread may add the free cubes'
   uint32_t flags = 0;            // creation flags (emissive list policy for edits)
   std::atomic<uint64_t> generation{0};   // bumped by edits that move device buffers
-  // free cubes (vt_internal.h), built by the first render of the scene
+  // free cubes (vt_internal.h), built by the first render of the scene, or the
+  // second where the first is a small edit-mode image (`shown`)
   std::atomic<unsigned long long*> runs{nullptr};
   std::atomic<bool> runs_tried{false};   // built, or not to be had
+  std::atomic<bool> shown{false};
   std::mutex runs_mu;            // held while they are built and while the bricks change
   std::vector<vt_material> host_palette;
   // the reference's flat material table and the record offset of each
