@@ -180,3 +180,26 @@ def test_tuning_times_the_wavefront_and_leaves_the_form(wctx):
         assert wctx.launch_count() - n == 1
     finally:
         close_all(job, scene, env)
+
+
+@pytest.mark.parametrize("w,h,jobs,block", [(512, 512, 2, True), (512, 513, 2, False), (1024, 513, 1, True), (256, 256, 8, True),
+                                            (256, 257, 8, False)])
+def test_several_jobs_leave_the_block_form_earlier(wctx, w, h, jobs, block):
+    """Launches of several jobs take the block form up to 2^18 samples a round
+    (two rounds here); the images are the wavefront's."""
+    made = [gpu_setup(wctx, config(w, h, bounces=0, seed=30 + k)) for k in range(jobs)]
+    js = [m[2] for m in made]
+    try:
+        wctx.render_batch(js, 1, kernel=2)
+        want = [j.readback().view(np.uint32) for j in js]
+        for j in js:
+            j.reset()
+        n = wctx.launch_count()
+        wctx.render_batch(js, 1)
+        n = wctx.launch_count() - n
+        assert n == 2 if block else n > 8
+        for j, a in zip(js, want):
+            assert np.array_equal(j.readback().view(np.uint32), a)
+    finally:
+        for sc, env, j in made:
+            close_all(j, sc, env)

@@ -1575,6 +1575,17 @@ static bool eye_inside(const Frame& F) {
   return in;
 }
 
+// Launches of several jobs, whose block form spills twice as much (the job's
+// record is in registers or a table): up to kBlockJobItems samples a round.
+// Block against wavefront, us, 2 to 9 jobs over spheres of 32-100^3: two bounces,
+// 0.8 M samples 330 / 373, 1.2 M 442 / 445, 1.8 M 598 / 556, 3.5 M 1006 / 840;
+// five, 1.2 M 570 / 687, 1.8 M 757 / 807; 20 jobs, five bounces, 1.8 M 839 / 851.
+constexpr int64_t kBlockJobItems = 1 << 18;
+
+static bool block_form(int64_t items, int64_t rounds, size_t jobs, int64_t inside) {
+  return items * rounds <= kBlockWork && inside <= kBlockInside && (jobs == 1 || items <= rounds * kBlockJobItems);
+}
+
 // A launch of at most kPathsItems samples: one kernel over the samples, then
 // the accumulation; a single pass of one job accumulates as it goes.
 static int paths_launch(vt_context* ctx, const std::vector<JobEntry>& entries, int64_t items) {
@@ -1914,7 +1925,7 @@ int vt::render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const 
       rc = paths_launch(ctx, entries, items);
       if (rc == VT_OK && foreign) VT_CUDA(cudaStreamSynchronize(ctx->stream), "samples");
       wave = false;
-    } else if (by_size && items * (max_b + 2) <= kBlockWork && inside <= kBlockInside) {
+    } else if (by_size && block_form(items, max_b + 2, entries.size(), inside)) {
       rc = block_launch(ctx, entries, grids, items);
       wave = rc == VT_EBUDGET || rc == VT_ENOMEM;
     }
