@@ -438,14 +438,14 @@ VT_API int vt_job_set_integrator(vt_job* job, int32_t integrator);
  * receives VT_SAMPLES_PENDING or VT_FINISHED_RENDERING.  The call queues GPU
  * work and returns; vt_job_synchronize or a readback waits for it.
  *
- * The first render of a scene, by this or any other call that renders (a
- * server's too), looks for empty cubes of its 4x4x4 bricks that rays can
- * cross in one step.  A scene open enough for them to pay keeps them in eight
- * bytes a brick (137 MB for 1024^3), counted in its device_bytes and in
- * vt_context_memory from then on; the search itself takes up to one byte a
- * brick of working memory, returned at once.  There are none for scenes of a
- * context with a budget, for volumes that a server with a budget keeps, and
- * where the memory is not to be had; images are the same without. */
+ * The first render of a scene, by this call, vt_render_batch or a server, looks
+ * for empty cubes of its 4x4x4 bricks that rays can cross in one step; where it
+ * is a small edit-mode image, the second one does.  A scene open enough for
+ * them to pay keeps them in eight bytes a brick (137 MB for 1024^3), counted in
+ * its device_bytes and in vt_context_memory from then on; the search itself
+ * takes about a byte a brick of working memory, returned at once.  There are
+ * none for scenes of a context with a budget, for volumes that a server with a
+ * budget keeps, and where the memory is not to be had; images are the same. */
 VT_API int vt_job_render(vt_job* job, int32_t passes, int32_t* result);
 VT_API int vt_job_synchronize(vt_job* job);
 VT_API int vt_job_sample_count(const vt_job* job, int32_t* samples);
@@ -517,17 +517,19 @@ VT_API int vt_job_remove_voxel(vt_job* job, float x, float y, int32_t restart,
                                int32_t voxel[3]);
 
 /* ------------------------------------------------------------- batching -- */
-/* Trace `passes` samples per pixel for every job in one wavefront launch:
- * path slots pull (job, pass, pixel) work items from a device counter and
- * rounds of shading and DDA kernels run over all jobs' paths at once,
- * instead of one launch per job and pass.  Results are identical to rendering
- * each job alone (counter-based random streams, per-pixel sample order).
- * opts may be NULL (context defaults). */
+/* Trace `passes` samples per pixel for every job in one launch, instead of one
+ * per job and pass: by default a thread per sample or block wavefronts for few
+ * samples (vt_diag_set_kernel), and otherwise, or where path_slots,
+ * blocks_per_sm or kernel 2 is given, the wavefront, whose path slots pull
+ * (job, pass, pixel) work items from a device counter and whose rounds of
+ * shading and DDA kernels run over all jobs' paths at once.  Results are
+ * identical to rendering each job alone (counter-based random streams,
+ * per-pixel sample order).  opts may be NULL (context defaults). */
 typedef struct vt_batch_opts {
-  int32_t path_slots;      /* paths in flight per launch, 0 = context default (8M) */
+  int32_t path_slots;      /* wavefront with as many paths in flight, 0 = by size, 8M */
   int32_t blocks_per_sm;   /* resident blocks per SM, 0 = auto                  */
   int32_t threads_per_block; /* 0 = auto                                        */
-  int32_t kernel;          /* 0 = auto, 1 = plain per-pixel, 2 = wavefront      */
+  int32_t kernel;          /* 0 = the context's, 1 = plain per-pixel, 2 = wavefront */
 } vt_batch_opts;
 VT_API int vt_render_batch(vt_context* ctx, vt_job* const* jobs, int32_t n_jobs,
                            int32_t passes, const vt_batch_opts* opts,

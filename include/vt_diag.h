@@ -56,7 +56,9 @@ VT_API int vt_diag_render_counted(vt_job* job, int32_t passes, uint64_t* counter
 VT_API int vt_diag_set_kernel(vt_context* ctx, int32_t kernel);
 
 /* Wavefront rounds replayed as a captured CUDA graph (enabled = 1, the
- * default) or launched one by one (0).  Results are identical. */
+ * default) or launched one by one (0).  A launch whose samples all have a slot
+ * runs its rounds once and launches them one by one in either case.  Results
+ * are identical. */
 VT_API int vt_diag_set_graphs(vt_context* ctx, int32_t enabled);
 
 /* Wavefront lanes: 2 (the default) runs two independent wavefronts over the

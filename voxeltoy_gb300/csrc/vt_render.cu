@@ -782,8 +782,9 @@ __global__ void __launch_bounds__(256, 4) k_wf_trace_pool(const WfParams P, cons
 // bounces): four kernels a round and lane, most of them a few microseconds.
 // Here a round costs its block three barriers.  Per sample the block form is
 // the slower one: all four parts run at the registers of the largest (64, 1024
-// threads an SM), and a block of a thousand paths ends every DDA part waiting
-// for its longest segments.  Measured (us, thread per sample / block /
+// threads an SM, with spills of 256 bytes a thread for one job and 480 to 588
+// for a table of jobs), and a block of a thousand paths ends every DDA part
+// waiting for its longest segments.  Measured (us, thread per sample / block /
 // wavefront; the line to the wavefront is drawn in vt_api.cu, with more):
 //   19 k samples of 64^3 spheres          118 /  170 /    -
 //   262 k of 128^3 noise, 8 bounces       610 /  462 /  761

@@ -172,11 +172,12 @@ int fixed_scratch_setup(int device);
 // Rebuilds a job's frame when its scene was edited since (scene->generation).
 int refresh_job(vt_job* j);
 // passes[i] samples per pixel for jobs[i]; kernel 1 = plain, 2 = wavefront,
-// 0 = the wavefront, or for few samples a thread per sample.
+// 0 = by the launch's size (render_wavefront's by_size).
 int render_jobs(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32_t* passes, int kernel,
                 int tile_pixels, int blocks_per_sm, bool count);
 // Wavefront form; `slots` path slots per launch (0 = context default).
-// by_size: launches of few samples take a thread per sample instead.
+// by_size: a launch of few samples takes a thread per sample instead, one of
+// more a block wavefront (k_paths_block), up to the lines beside kPathsItems.
 int render_wavefront(vt_context* ctx, vt_job* const* jobs, int32_t n, const int32_t* passes, int slots,
                      int blocks_per_sm, bool count, bool by_size);
 }  // namespace vt
