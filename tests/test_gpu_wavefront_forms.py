@@ -134,12 +134,14 @@ def test_back_to_the_defaults(wctx):
     finally:
         close_all(job, scene, env)
 
-@pytest.mark.parametrize("w,h,inside,block", [(768, 512, True, True), (769, 512, True, False), (769, 512, False, True),
-                                              (480, 270, True, True)])
-def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, inside, block):
+@pytest.mark.parametrize("w,h,bounces,inside,block", [
+    (768, 512, 3, True, True), (769, 512, 3, True, False), (769, 512, 3, False, True), (480, 270, 3, True, True),
+    (768, 512, 2, True, True), (769, 512, 2, True, False), (1024, 768, 1, True, True), (1025, 768, 1, True, False),
+    (1536, 1024, 0, True, True), (1537, 1024, 0, True, False)])
+def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, bounces, inside, block):
     """A launch by size takes one kernel and the accumulation (a single pass of
     few samples one kernel), or the wavefront's; the images are the same."""
-    cfg = config(w, h, bounces=3)
+    cfg = config(w, h, bounces=bounces)
     if inside:
         cfg.voxels = np.ones((24, 24, 24), np.uint8)
         cfg.voxels[3:-3, 3:-3, 3:-3] = 0
@@ -159,7 +161,8 @@ def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, insi
         n = wctx.launch_count()
         wctx.render_batch([job, other], 1)            # both cameras count
         n = wctx.launch_count() - n
-        assert n == (2 if not inside or w * h + 1200 <= 3 << 17 else rounds)
+        line = max(3 << 17, (3 << 19) >> bounces) if inside else 1 << 30
+        assert n == (2 if w * h + 1200 <= min(line, (bounces + 2) << 18) else rounds)
         assert np.array_equal(job.readback().view(np.uint32), want)
     finally:
         close_all(other, job, scene, env)

@@ -1565,6 +1565,9 @@ constexpr int64_t kBlockWork = 16 << 20;
 // 393 k 1022 / 919 and 1975 / 1696, 1.05 M 2242 / 1690 and 4348 / 3243; a hollow
 // in 128^3 noise, 393 k 729 / 760 and 1138 / 1257, 614 k 1049 / 917 and
 // 1595 / 1487; an empty 48^3 room, four bounces, 320 k 540 / 636, 614 k 924 / 898.
+// With one bounce or none the rounds are few, and the line lies two and four
+// times as far: the 128^3 room, one bounce, 786 k 519 / 521; the empty one, none,
+// 1.05 M 164 / 190, 2.1 M 295 / 283.
 // Seen from outside, a 64^3 box with its front open, 1.05 M 1144 / 1039 and
 // 1635 / 1578.
 constexpr int64_t kBlockInside = 3 << 17;
@@ -1583,7 +1586,7 @@ static bool eye_inside(const Frame& F) {
 constexpr int64_t kBlockJobItems = 1 << 18;
 
 static bool block_form(int64_t items, int64_t rounds, size_t jobs, int64_t inside) {
-  return items * rounds <= kBlockWork && inside <= kBlockInside && (jobs == 1 || items <= rounds * kBlockJobItems);
+  return items * rounds <= kBlockWork && inside <= std::max(kBlockInside, 4 * kBlockInside >> (rounds - 2)) && (jobs == 1 || items <= rounds * kBlockJobItems);
 }
 
 // A launch of at most kPathsItems samples: one kernel over the samples, then
