@@ -137,7 +137,7 @@ def test_back_to_the_defaults(wctx):
 @pytest.mark.parametrize("w,h,bounces,inside,block", [
     (768, 512, 3, True, True), (769, 512, 3, True, False), (769, 512, 3, False, True), (480, 270, 3, True, True),
     (768, 512, 2, True, True), (769, 512, 2, True, False), (1024, 768, 1, True, True), (1025, 768, 1, True, False),
-    (1536, 1024, 0, True, True), (1537, 1024, 0, True, False)])
+    (1536, 1024, 0, True, True), (1537, 1024, 0, True, False), (769, 512, 64, False, False), (513, 300, 64, True, True)])
 def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, bounces, inside, block):
     """A launch by size takes one kernel and the accumulation (a single pass of
     few samples one kernel), or the wavefront's; the images are the same."""
@@ -159,10 +159,16 @@ def test_cameras_inside_the_volume_leave_the_block_form_earlier(wctx, w, h, boun
         assert np.array_equal(job.readback().view(np.uint32), want)
         job.reset()
         n = wctx.launch_count()
+        wctx.render_batch([job, other], 1, kernel=2)
+        n_all = wctx.launch_count() - n
+        job.reset()
+        other.reset()
+        n = wctx.launch_count()
         wctx.render_batch([job, other], 1)            # both cameras count
         n = wctx.launch_count() - n
         line = max(3 << 17, (3 << 19) >> bounces) if inside else 1 << 30
-        assert n == (2 if w * h + 1200 <= min(line, (bounces + 2) << 18) else rounds)
+        small = (w * h + 1200) * (bounces + 2) <= 16 << 20
+        assert n == (2 if small and w * h + 1200 <= min(line, (bounces + 2) << 18) else n_all)
         assert np.array_equal(job.readback().view(np.uint32), want)
     finally:
         close_all(other, job, scene, env)

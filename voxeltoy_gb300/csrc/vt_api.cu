@@ -1586,7 +1586,8 @@ static bool eye_inside(const Frame& F) {
 constexpr int64_t kBlockJobItems = 1 << 18;
 
 static bool block_form(int64_t items, int64_t rounds, size_t jobs, int64_t inside) {
-  return items * rounds <= kBlockWork && inside <= std::max(kBlockInside, 4 * kBlockInside >> (rounds - 2)) && (jobs == 1 || items <= rounds * kBlockJobItems);
+  const int64_t inside_line = rounds == 2 ? 4 * kBlockInside : (rounds == 3 ? 2 * kBlockInside : kBlockInside);
+  return items * rounds <= kBlockWork && inside <= inside_line && (jobs == 1 || items <= rounds * kBlockJobItems);
 }
 
 // A launch of at most kPathsItems samples: one kernel over the samples, then
